@@ -15,10 +15,10 @@ cudaError_t launch_offsets_from_sizes(const int32_t*, int32_t*, int64_t, int64_t
 cudaError_t launch_permute(const void*, const int32_t*, void*, int64_t, int64_t, int64_t, int64_t, bool, cudaStream_t);
 cudaError_t launch_block_map(const void*, const void*, const int32_t*, uint8_t*, int64_t, int64_t, int64_t, float,
                              const int32_t*, const int32_t*, cudaStream_t);
-cudaError_t launch_build_runs(const uint8_t*, const int32_t*, int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
-cudaError_t launch_build_qtiles(const int32_t*, int4*, int32_t*, int64_t, int64_t, int64_t, int, cudaStream_t);
+cudaError_t launch_attn_lists(const int32_t*, int4*, int32_t*, const uint8_t*, const int32_t*, int2*, int32_t*, int32_t*, int32_t*,
+                              int64_t, int64_t, int64_t, int64_t, int, int, bool, bool, cudaStream_t);
 cudaError_t launch_sparse_attn_tc(const void*, const void*, const void*, void*, const int32_t*, const int4*,
-                                  const int32_t*, const int2*, const int32_t*, int32_t*, int64_t, int64_t, int64_t,
+                                  const int32_t*, const int32_t*, const int2*, const int32_t*, int32_t*, int64_t, int64_t, int64_t,
                                   int64_t, float, void* const*, const int32_t*, int, int64_t, int, float*, cudaStream_t,
                                   const uint8_t* ear_map = nullptr, const int32_t* ear_k_offsets = nullptr,
                                   int ear_max_runs = 0);
@@ -29,8 +29,6 @@ cudaError_t launch_ear_scores(const void*, const void*, const void*, const int32
                               cudaStream_t);
 cudaError_t launch_ear_select(const float*, const float*, const int32_t*, const int32_t*, uint8_t*, int64_t, int64_t, int64_t,
                               float, const int32_t*, const int32_t*, cudaStream_t);
-cudaError_t launch_ear_build_runs(const uint8_t*, const int32_t*, int2*, int32_t*, int64_t, int64_t, int64_t, int64_t, int,
-                                  cudaStream_t);
 cudaError_t launch_euclid_assign_tc(const void*, const void*, float*, int32_t*, int2*, int32_t*, int64_t, int64_t, int64_t,
                                     int32_t*, cudaStream_t);
 cudaError_t launch_append_text_blocks(const uint8_t*, const int32_t*, const int32_t*, const int32_t*, const int32_t*,
@@ -300,13 +298,15 @@ static int sparse_attn_impl(bool tensor_core, const void* q, const void* k, cons
   int32_t* nruns = ws_at<int32_t>(workspace, w.nruns);
   int4* qtiles = ws_at<int4>(workspace, w.qtiles);
   int32_t* nqtiles = ws_at<int32_t>(workspace, w.nqtiles);
-  int32_t* status = ws_at<int32_t>(workspace, w.status);
-  SVOO_CUDA(launch_build_runs(map, k_offsets, runs, nruns, BH, QC, KC, st));
-  SVOO_CUDA(launch_build_qtiles(q_offsets, qtiles, nqtiles, BH, S, QC, tensor_core ? 256 : 128, st));
+  int32_t* head_order = ws_at<int32_t>(workspace, w.head_order);
+  int32_t* sched = ws_at<int32_t>(workspace, w.sched);
+  int32_t* status = ws_at<int32_t>(workspace, w.status);            // word 0: attention kernel
+  SVOO_CUDA(cudaMemsetAsync(sched, 0, (size_t)(w.status - w.sched) + 4, st));
+  SVOO_CUDA(launch_attn_lists(q_offsets, qtiles, nqtiles, map, k_offsets, runs, nruns, sched, head_order, BH, S, QC, KC, max_runs(KC),
+                              tensor_core ? 256 : 128, tensor_core && single_tile_kernel_wins(S, QC), false, st));
   if (tensor_core) {
-    SVOO_CUDA(cudaMemsetAsync(status, 0, 4, st));                     // word 0: attention kernel
-    SVOO_CUDA(launch_sparse_attn_tc(q, k, v, out, out_row_idx, qtiles, nqtiles, runs, nruns, status, BH, S, QC, KC,
-                                    sm_scale, peer_dst, my_heads, world, n_loc, H, lse, st));
+    SVOO_CUDA(launch_sparse_attn_tc(q, k, v, out, out_row_idx, qtiles, nqtiles, head_order, runs, nruns, status, BH, S, QC,
+                                    KC, sm_scale, peer_dst, my_heads, world, n_loc, H, lse, st));
   } else {
     SVOO_CUDA(launch_sparse_attn_mma(q, k, v, out, out_row_idx, qtiles, nqtiles, runs, nruns, BH, S, QC, KC, sm_scale,
                                      st));
@@ -352,7 +352,7 @@ int svoo_b200_sparse_attn_simt(const void* q, const void* k, const void* v, cons
 // ---------------------------------------------------------------------------------------
 namespace {
 struct EarWorkspace {
-  int64_t vnorm, cvd, vcsq, runs, nruns, qtiles, nqtiles, status, total;
+  int64_t vnorm, cvd, vcsq, runs, nruns, qtiles, nqtiles, head_order, sched, status, total;
 };
 inline int ear_max_runs(int64_t KC) { return (int)(KC / 2 + 4); }   // token runs + the centroid run + sentinel
 inline EarWorkspace ear_layout(int64_t BH, int64_t N, int64_t QC, int64_t KC) {
@@ -365,7 +365,9 @@ inline EarWorkspace ear_layout(int64_t BH, int64_t N, int64_t QC, int64_t KC) {
   w.runs = take(BH * QC * (int64_t)ear_max_runs(KC) * 8);
   w.nruns = take(BH * QC * 4);
   w.qtiles = take(BH * (int64_t)max_qtiles(N, QC) * 16);
-  w.nqtiles = take(BH * 4);
+  w.nqtiles = take(BH * 8);
+  w.head_order = take(BH * 4);
+  w.sched = take((BH + 1) * 4);
   w.status = take(16);
   w.total = o;
   return w;
@@ -448,12 +450,14 @@ static int sparse_attn_ear_impl(const void* q, const void* k_ext, const void* v_
   int32_t* nruns = ws_at<int32_t>(ear_workspace, w.nruns);
   int4* qtiles = ws_at<int4>(ear_workspace, w.qtiles);
   int32_t* nqtiles = ws_at<int32_t>(ear_workspace, w.nqtiles);
+  int32_t* head_order = ws_at<int32_t>(ear_workspace, w.head_order);
+  int32_t* sched = ws_at<int32_t>(ear_workspace, w.sched);
   int32_t* status = ws_at<int32_t>(ear_workspace, w.status);
-  SVOO_CUDA(launch_ear_build_runs(map, k_offsets, runs, nruns, BH, S, QC, KC, ear_max_runs(KC), st));
-  SVOO_CUDA(launch_build_qtiles(q_offsets, qtiles, nqtiles, BH, S, QC, 256, st));
-  SVOO_CUDA(cudaMemsetAsync(status, 0, 4, st));
-  SVOO_CUDA(launch_sparse_attn_tc(q, k_ext, v_ext, out, out_row_idx, qtiles, nqtiles, runs, nruns, status, BH, S, QC, KC,
-                                  sm_scale, peer_dst, my_heads, world, n_loc, H, lse, st, map, k_offsets, ear_max_runs(KC)));
+  SVOO_CUDA(cudaMemsetAsync(sched, 0, (size_t)(w.status - w.sched) + 4, st));
+  SVOO_CUDA(launch_attn_lists(q_offsets, qtiles, nqtiles, map, k_offsets, runs, nruns, sched, head_order, BH, S, QC, KC, ear_max_runs(KC), 256,
+                              single_tile_kernel_wins(S, QC), true, st));
+  SVOO_CUDA(launch_sparse_attn_tc(q, k_ext, v_ext, out, out_row_idx, qtiles, nqtiles, head_order, runs, nruns, status, BH, S, QC,
+                                  KC, sm_scale, peer_dst, my_heads, world, n_loc, H, lse, st, map, k_offsets, ear_max_runs(KC)));
   return SVOO_OK;
 }
 

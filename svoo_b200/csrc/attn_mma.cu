@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(256, 1) sparse_attn_mma_kernel(
     float scale_log2) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int bh = blockIdx.y;
-  if ((int)blockIdx.x >= nqtiles[bh]) return;
+  if ((int)blockIdx.x >= nqtiles[2 * bh]) return;
   const int4 tile = qtiles[(int64_t)bh * max_tiles + blockIdx.x];
   const int qi = tile.x, row0 = tile.y, row1 = tile.z;
   const int nr = nruns[(int64_t)bh * QC + qi];

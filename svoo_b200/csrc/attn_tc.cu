@@ -9,8 +9,9 @@
 //   warps 0-3   softmax of query tile 0: thread r owns row r (TMEM lane r).  The 128 scores of the
 //   warps 4-7   row are copied to registers and S is handed back at once; row max, exp2, row sum,
 //               P packed to bf16 into the tile's own TMEM columns; same for query tile 1
-//   warp 8      TMA producer for Q (once) and K, warp 9 for V: cp.async.bulk.tensor 2-D boxes of
-//               64 columns with the 128-byte swizzle, no multicast; two-stage rings for K and V
+//   warp 8      producer of Q (once) and K, warp 9 of V: cp.async.bulk.tensor 2-D boxes of
+//               64 columns with the 128-byte swizzle, no multicast; two-stage rings for K and V.
+//               kGather: a tile of many short runs is copied row by row with cp.async instead
 //   warp 10     MMA issuer (one elected thread): S = Q_w K^T into TMEM (tcgen05.mma, both
 //               operands from shared memory), then O_w += P_w V with P_w read from TMEM
 //   warp 11     idle; it completes the service warpgroup, which gives registers to the softmax
@@ -27,7 +28,7 @@
 // TMEM columns (512 allocated): S [0,128)  P0 [128,192)  P1 [192,256)  O0 [256,384)  O1 [384,512).
 // Semantics: svoo/co_clustering.py:949-1108 (scale D^-0.5, zero output without keys).
 #include <type_traits>
-#include "tc_common.cuh"
+#include "attn_common.cuh"
 
 namespace svoo {
 namespace tc {
@@ -55,6 +56,10 @@ constexpr int kThreads = 12 * 32;       // warp 11 only completes the service wa
 #define SVOO_REGS_SERVICE 104        // 128 * 104 + 256 * 200 = 64512 = the 12 warps' launch allotment
 #endif
 constexpr int kRegsService = SVOO_REGS_SERVICE, kRegsSoftmax = 200;
+// kGather: a tile of more TMA boxes than this (both halves counted) is gathered with cp.async instead.
+// Measured on a 12 x 20,280 layer with 500 key clusters (18 boxes per tile): 823 us with TMA alone, 763 / 753 /
+// 750 / 792 us with limits 6 / 10 / 16 / 24.
+constexpr int kMaxBoxes = 16;
 constexpr int kBoxHeights = 8;                           // TMA boxes of 1, 2, 4, ..., 128 rows
 
 // Tensor maps of one launch: Q with 128-row boxes; K and V with one map per box height, so a
@@ -64,58 +69,10 @@ struct AttnMaps {
   CUtensorMap k[kBoxHeights];
   CUtensorMap v[kBoxHeights];
 };
-// Optional destination of the output rows on other GPUs: row n of local head bh goes to rank
-// n / n_loc, row n % n_loc, head head[bh] of that rank's [n_loc, H, 128] array.  n_loc == 0: the
-// rows go to `out` of this GPU.
-struct OutPeers {
-  bf16* dst[16];
-  int n_loc;
-  int H;
-  int16_t head[128];
-};
-constexpr float kRescaleThreshold = 8.0f;
 
 enum Bar { Q_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, S_FULL = 9, P_READY = 11, P_FREE = 13, S_FREE = 15, NUM_BARS = 17 };
 // TMEM columns: one S accumulator shared by the two query tiles, then P0, P1 (packed bf16), O0, O1.
 constexpr uint32_t kColS = 0, kColP = 128, kColO = 256;
-
-// Packed fp32 pairs (one instruction for two lanes of data): x = s * scale + neg_m and the
-// running pair of row sums.
-__device__ __forceinline__ void fma2(float& x0, float& x1, uint32_t a0, uint32_t a1, uint64_t scale2, uint64_t negm2) {
-  asm("{\n\t.reg .b64 a, x;\n\t"
-      "mov.b64 a, {%2, %3};\n\t"
-      "fma.rn.f32x2 x, a, %4, %5;\n\t"
-      "mov.b64 {%0, %1}, x;\n\t}\n"
-      : "=f"(x0), "=f"(x1) : "r"(a0), "r"(a1), "l"(scale2), "l"(negm2));
-}
-__device__ __forceinline__ void add2(uint64_t& acc, float p0, float p1) {
-  asm("{\n\t.reg .b64 p;\n\t"
-      "mov.b64 p, {%1, %2};\n\t"
-      "add.rn.f32x2 %0, %0, p;\n\t}\n"
-      : "+l"(acc) : "f"(p0), "f"(p1));
-}
-__device__ __forceinline__ uint64_t pair2(float v) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-  return r;
-}
-__device__ __forceinline__ float pair_sum(uint64_t acc) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(acc));
-  return a + b;
-}
-// 16 columns: p = exp2(s * scale + neg_m) -> 8 packed bf16 pairs, row sums into `acc`.
-__device__ __forceinline__ void exp_pack16(const uint32_t (&r)[16], uint32_t* pk, uint64_t scale2, uint64_t negm2,
-                                           uint64_t& acc) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float x0, x1;
-    fma2(x0, x1, r[2 * i], r[2 * i + 1], scale2, negm2);
-    const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-    add2(acc, p0, p1);
-    pk[i] = pack_bf16x2(p0, p1);
-  }
-}
 
 // Shared-memory matrix descriptors, 128-byte swizzle, descriptor version 1 (sm_100).
 //   K-major  (Q, K: rows = M/N index, 64 contiguous elements of the reduction dim per 128-byte row):
@@ -174,18 +131,20 @@ __device__ __forceinline__ void tma_gather_tile(uint32_t dst, const CUtensorMap*
 // that follow the tokens of all heads in K and V).  Centroid j is a virtual key standing for the whole
 // cluster j: it carries the additive bias log(|K_j| + 1e-6) (svoo/co_clustering.py:1873-1876) when the
 // cluster was pruned and -inf when its tokens are in the list themselves.
-template <bool kEar>
+template <bool kEar, bool kGather>
 __global__ void __launch_bounds__(kThreads, 1) sparse_attn_tc_kernel(
-    const __grid_constant__ AttnMaps maps, const __grid_constant__ OutPeers peers, bf16* __restrict__ out,
-    const int32_t* __restrict__ out_row_idx, const int4* __restrict__ qtiles, const int32_t* __restrict__ nqtiles,
-    const int2* __restrict__ runs, const int32_t* __restrict__ nruns, int S, int QC, int max_tiles, int max_runs,
-    float scale_log2, int32_t* __restrict__ status, float* __restrict__ lse, const uint8_t* __restrict__ map,
+    const __grid_constant__ AttnMaps maps, const __grid_constant__ OutPeers peers, const bf16* __restrict__ k_rows,
+    const bf16* __restrict__ v_rows, bf16* __restrict__ out, const int32_t* __restrict__ out_row_idx,
+    const int4* __restrict__ qtiles, const int32_t* __restrict__ nqtiles, const int32_t* __restrict__ head_order,
+    const int2* __restrict__ runs, const int32_t* __restrict__ nruns, int BH, int S, int QC, int max_tiles, int per_head,
+    int max_runs, float scale_log2, int32_t* __restrict__ status, float* __restrict__ lse, const uint8_t* __restrict__ map,
     const int32_t* __restrict__ k_offsets, int KC, int rows_total) {
   constexpr int kMaxRunsSmem = AttnSmem<kEar>::kMaxRuns;
   extern __shared__ unsigned char smem_raw[];
-  const int bh = blockIdx.y;
-  if ((int)blockIdx.x >= nqtiles[bh]) return;
-  const int4 tile = qtiles[(int64_t)bh * max_tiles + blockIdx.x];
+  pdl_trigger();                                       // the single-tile kernel may fill the SMs that this grid leaves
+  int bh, t_idx;
+  if (!pick_tile<1>((int)blockIdx.x, BH, per_head, nqtiles, head_order, 0, bh, t_idx)) return;
+  const int4 tile = qtiles[(int64_t)bh * max_tiles + t_idx];
   const int qi = tile.x, row0 = tile.y, row1 = tile.z;
   const int nr = min(nruns[(int64_t)bh * QC + qi], kMaxRunsSmem - 1);
   const int2* rl = runs + ((int64_t)bh * QC + qi) * max_runs;
@@ -251,24 +210,65 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_tc_kernel(
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsService));
   if (warp == kKWarp || warp == kVWarp) {
     // ---------------------------------------------------------------- TMA producers (K + Q, V)
-    if (lane == 0 && T > 0) {
-      const int is_v = warp == kVWarp;
-      if (!is_v) {
-        mbar_expect_tx(bar(Q_FULL), nq * kTile);
-        for (int w = 0; w < nq; ++w)
-          for (int h = 0; h < 2; ++h)
-            tma_load_2d(q_s + w * kTile + h * kBox, &maps.q, h * 64, bh * S + row0 + w * kBM, bar(Q_FULL));
-      }
-      const CUtensorMap* tm = is_v ? maps.v : maps.k;
-      const uint32_t stage0 = is_v ? v_s : k_s;
-      const int full = is_v ? V_FULL : K_FULL, empty = is_v ? V_EMPTY : K_EMPTY;
+    const bool is_v = warp == kVWarp;
+    if (!is_v && lane == 0 && T > 0) {
+      mbar_expect_tx(bar(Q_FULL), nq * kTile);
+      for (int w = 0; w < nq; ++w)
+        for (int h = 0; h < 2; ++h)
+          tma_load_2d(q_s + w * kTile + h * kBox, &maps.q, h * 64, bh * S + row0 + w * kBM, bar(Q_FULL));
+    }
+    const CUtensorMap* tm = is_v ? maps.v : maps.k;
+    const uint32_t stage0 = is_v ? v_s : k_s;
+    const int full = is_v ? V_FULL : K_FULL, empty = is_v ? V_EMPTY : K_EMPTY;
+    if constexpr (!kGather) {
       int r_cur = 0;
-      for (int j = 0; j < T; ++j) {
+      for (int j = 0; lane == 0 && j < T; ++j) {
         const int s = j & 1;
         if (!mbar_wait(bar(empty + s), ((j >> 1) & 1) ^ 1, abort_flag)) break;
         mbar_expect_tx(bar(full + s), kTile);
         tma_gather_tile(stage0 + s * kTile, tm, runs_s, nr, r_cur, j, L, bh * S, rows_total, bar(full + s));
       }
+    } else {
+      const int chunk = lane & 15;
+      const bf16* src_base = (is_v ? v_rows : k_rows) + (int64_t)bh * S * kHeadDim + chunk * 8;
+      int cur = 0, pending = -1;                           // pending: stage whose cp.async copies are not reported yet
+      auto report = [&]() {
+        cp_async_wait<0>();
+        fence_async_proxy();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(full + pending));
+        pending = -1;
+      };
+      for (int j = 0; j < T; ++j) {
+        const int s = j & 1, v0 = j * kBN;
+        const uint32_t par = ((j >> 1) & 1) ^ 1;
+        if (pending >= 0) report();
+        if (!__all_sync(0xffffffffu, mbar_wait(bar(empty + s), par, abort_flag))) break;
+        advance_run(runs_s, nr, v0, lane, cur);
+        // boxes of this tile if TMA fetches it (lane l: run cur + l)
+        const int n = min(cur + lane, nr), begin = runs_s[n].y, end = runs_s[min(n + 1, nr)].y;
+        const int len = max(min(end, v0 + kBN) - max(begin, v0), 0);
+        int boxes = 2 * (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc((unsigned)len));
+        if (__any_sync(0xffffffffu, lane == 31 && end < min(v0 + kBN, L))) boxes = kMaxBoxes + 1;   // more than 32 runs
+        if (boxes <= kMaxBoxes) {
+          if (lane == 0) {
+            int r_cur = cur;
+            mbar_expect_tx(bar(full + s), kTile);
+            tma_gather_tile(stage0 + s * kTile, tm, runs_s, nr, r_cur, j, L, bh * S, rows_total, bar(full + s));
+          }
+          __syncwarp();
+        } else {
+          const uint32_t dst = stage0 + s * kTile + (chunk >> 3) * kBox;
+#pragma unroll 1
+          for (int g = 0; g < kBN / 32; ++g) {
+            const int src = gather_source(runs_s, nr, L, v0 + g * 32, lane, cur);
+            gather_rows32(dst, src_base, src, g * 32, lane);
+          }
+          cp_async_commit();
+          pending = s;
+        }
+      }
+      if (pending >= 0) report();
     }
   } else if (warp == kMmaWarp) {
     // ---------------------------------------------------------------- MMA issuer
@@ -481,13 +481,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_tc_kernel(
       int dst = row;
       if (store && out_row_idx) dst = out_row_idx[(int64_t)bh * S + row];
       dst = store ? min(max(dst, 0), S - 1) : 0;
-      bf16* orow;
-      if (peers.n_loc == 0) {
-        orow = out + ((int64_t)bh * S + dst) * kHeadDim;
-      } else {                                           // store straight into the owning rank's sequence shard
-        const int p = dst / peers.n_loc;
-        orow = peers.dst[p] + ((int64_t)(dst - p * peers.n_loc) * peers.H + peers.head[bh]) * kHeadDim;
-      }
+      bf16* orow = out_row(peers, out, bh, S, dst);
       // log2 of the softmax denominator, sum_j 2^(s_j * scale * log2 e); -inf for a row without keys
       if (lse && store && (T == 0 || ok))
         lse[(int64_t)bh * S + dst] = (T == 0 || !(l_sum > 0.f)) ? -INFINITY : m_used + __log2f(l_sum);
@@ -530,8 +524,12 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_tc_kernel(
 }  // namespace tc
 
 
+cudaError_t launch_sparse_attn_small(const CUtensorMap&, const tc::OutPeers&, const void*, const void*, void*, const int32_t*,
+                                     const int4*, const int32_t*, const int32_t*, const int2*, const int32_t*, int32_t*, int64_t, int64_t,
+                                     int64_t, int64_t, int, float, float*, cudaStream_t, const uint8_t*, const int32_t*, bool);
+
 cudaError_t launch_sparse_attn_tc(const void* q, const void* k, const void* v, void* out, const int32_t* out_row_idx,
-                                  const int4* qtiles, const int32_t* nqtiles, const int2* runs, const int32_t* nruns,
+                                  const int4* qtiles, const int32_t* nqtiles, const int32_t* head_order, const int2* runs, const int32_t* nruns,
                                   int32_t* status, int64_t BH, int64_t S, int64_t QC, int64_t KC, float sm_scale,
                                   void* const* peer_dst, const int32_t* my_heads, int world, int64_t n_loc, int H,
                                   float* lse, cudaStream_t st, const uint8_t* ear_map, const int32_t* ear_k_offsets,
@@ -554,26 +552,29 @@ cudaError_t launch_sparse_attn_tc(const void* q, const void* k, const void* v, v
   for (int i = 0; i < tc::kBoxHeights && ok; ++i)
     ok = tc::make_row_tensor_map(&maps.k[i], k, kv_rows, 1 << i) && tc::make_row_tensor_map(&maps.v[i], v, kv_rows, 1 << i);
   if (!ok) return cudaErrorInvalidValue;
-  dim3 grid((unsigned)max_qtiles(S, QC), (unsigned)BH);
   const float scale_log2 = sm_scale * 1.4426950408889634f;
-  cudaError_t e;
-  if (ear) {
-    e = cudaFuncSetAttribute(tc::sparse_attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             tc::AttnSmem<true>::kBytes);
+  const int runs_per_row = ear ? ear_max_runs : max_runs(KC);
+  if (peer_dst) lse = nullptr;
+  const bool split = single_tile_kernel_wins(S, QC);
+  // tiles per head: of at least 129 rows each, or a cluster's whole 256-row tiles and its remainder
+  const int per_head = (int)(split ? S / (tc::kBM + 1) : S / (2 * tc::kBM) + QC);
+  if (per_head > 0) {
+    const bool gather = short_key_runs(S, KC);
+    auto* kernel = ear ? (gather ? &tc::sparse_attn_tc_kernel<true, true> : &tc::sparse_attn_tc_kernel<true, false>)
+                       : (gather ? &tc::sparse_attn_tc_kernel<false, true> : &tc::sparse_attn_tc_kernel<false, false>);
+    const int smem = ear ? tc::AttnSmem<true>::kBytes : tc::AttnSmem<false>::kBytes;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    tc::sparse_attn_tc_kernel<true><<<grid, tc::kThreads, tc::AttnSmem<true>::kBytes, st>>>(
-        maps, peers, (bf16*)out, out_row_idx, qtiles, nqtiles, runs, nruns, (int)S, (int)QC, max_qtiles(S, QC), ear_max_runs,
-        scale_log2, status, peer_dst ? nullptr : lse, ear_map, ear_k_offsets, (int)KC, (int)kv_rows);
-  } else {
-    e = cudaFuncSetAttribute(tc::sparse_attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             tc::AttnSmem<false>::kBytes);
-    if (e != cudaSuccess) return e;
-    tc::sparse_attn_tc_kernel<false><<<grid, tc::kThreads, tc::AttnSmem<false>::kBytes, st>>>(
-        maps, peers, (bf16*)out, out_row_idx, qtiles, nqtiles, runs, nruns, (int)S, (int)QC, max_qtiles(S, QC), max_runs(KC),
-        scale_log2, status, peer_dst ? nullptr : lse, nullptr, nullptr, (int)KC, (int)kv_rows);
+    kernel<<<(unsigned)(BH * per_head), tc::kThreads, smem, st>>>(
+        maps, peers, (const bf16*)k, (const bf16*)v, (bf16*)out, out_row_idx, qtiles, nqtiles, head_order, runs, nruns, (int)BH, (int)S,
+        (int)QC, max_qtiles(S, QC), per_head, runs_per_row, scale_log2, status, lse, ear_map, ear_k_offsets, (int)KC,
+        (int)kv_rows);
+    count_launches(1);
+    e = cudaGetLastError();
+    if (e != cudaSuccess || !split) return e;
   }
-  count_launches(1);
-  return cudaGetLastError();
+  return launch_sparse_attn_small(maps.q, peers, k, v, out, out_row_idx, qtiles, nqtiles, head_order, runs, nruns, status, BH, S, QC, KC,
+                                  runs_per_row, scale_log2, lse, st, ear_map, ear_k_offsets, per_head > 0);
 }
 
 }  // namespace svoo

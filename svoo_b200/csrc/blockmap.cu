@@ -169,99 +169,161 @@ __global__ void __launch_bounds__(256, 2) block_map_kernel(const bf16* __restric
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The two index lists of the attention kernels, in one launch: blocks [0, BH) write the query tiles of
+// one head each, the blocks after them the key-row runs of eight (head, query cluster) rows each.
+// ---------------------------------------------------------------------------------------------
+// Query tiles of every non-empty query cluster, in cluster order; thread i owns clusters
+// [kPer i, kPer (i + 1)).  Tiles of kRows rows; with kSplit (kRows = 256) a remainder of up to 128 rows goes
+// to a list of its own (the last QC entries of the head's tiles, for attn_small.cu).
+constexpr int kListThreads = 256;
+template <int kRows, bool kSplit>
+__device__ void build_qtiles(const int32_t* __restrict__ off, int4* __restrict__ out, int32_t* __restrict__ counts, int QC,
+                             int max_tiles) {
+  constexpr int kPer = (SVOO_MAX_ATTN_CLUSTERS + kListThreads - 1) / kListThreads;
+  __shared__ unsigned long long warp_tot[kListThreads / 32];
+  const int i = threadIdx.x, lane = i % 32, warp = i / 32;
+  int b[kPer + 1];
+#pragma unroll
+  for (int u = 0; u <= kPer; ++u) b[u] = off[min(kPer * i + u, QC)];
+  auto single = [](int rows) { return (int)(kSplit && rows > 0 && (rows - 1) % kRows < kAttnBM); };
+  unsigned long long n = 0;                              // (whole tiles, single tiles) of this thread's clusters
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int rows = b[u + 1] - b[u], s1 = single(rows);
+    n += (unsigned long long)((rows + kRows - 1) / kRows - s1) | (unsigned long long)s1 << 32;
+  }
+  unsigned long long incl = n;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const unsigned long long o = __shfl_up_sync(0xffffffffu, incl, s);
+    if (lane >= s) incl += o;
+  }
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  unsigned long long before = incl - n, total = 0;
+#pragma unroll
+  for (int w = 0; w < kListThreads / 32; ++w) {
+    if (w < warp) before += warp_tot[w];
+    total += warp_tot[w];
+  }
+  int pos = (int)(before & 0xffffffffu), spos = max_tiles - QC + (int)(before >> 32);
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int rows = b[u + 1] - b[u], s1 = single(rows), nt = (rows + kRows - 1) / kRows - s1;
+    int r = b[u];
+    for (int t = 0; t < nt; ++t, ++pos, r += kRows)
+      if (pos < max_tiles) out[pos] = make_int4(kPer * i + u, r, min(r + kRows, b[u + 1]), 0);
+    if (s1) {
+      if (spos < max_tiles) out[spos] = make_int4(kPer * i + u, r, b[u + 1], 0);
+      ++spos;
+    }
+  }
+  if (i == 0) {
+    counts[0] = min((int)(total & 0xffffffffu), max_tiles);
+    counts[1] = min((int)(total >> 32), QC);
+  }
+}
+
 // One warp per (head, query cluster): maximal stretches of consecutive selected, non-empty
 // key clusters become runs of the cluster-ordered K/V.  Run r is stored as
 // (first_row, virtual_begin): virtual_begin is the number of selected key rows before it, so
 // the concatenation of all runs is addressed by one "virtual" row index; entry [nruns] is a
 // sentinel (0, total selected rows).
-__global__ void __launch_bounds__(256) build_runs_kernel(const uint8_t* __restrict__ map,
-                                                         const int32_t* __restrict__ k_offsets, int2* __restrict__ runs,
-                                                         int32_t* __restrict__ nruns, int QC, int KC, int max_runs,
-                                                         int rows_total) {
-  const int row = blockIdx.x * 8 + threadIdx.x / 32;
-  if (row >= rows_total) return;
+// kEar: the K/V tensors are the cluster-ordered rows of all heads followed by the centroid rows of all
+// heads ([BH*S + BH*KC, 128]), and the list ends with ONE more run, the KC centroid rows of the head
+// (the attention kernels mask the centroids of the selected clusters).
+template <bool kEar>
+__device__ void build_runs(const uint8_t* __restrict__ map, const int32_t* __restrict__ k_offsets, int2* __restrict__ runs,
+                           int32_t* __restrict__ nruns, int32_t* __restrict__ head_work, int row, int BH, int S, int QC, int KC,
+                           int max_runs) {
   const int lane = threadIdx.x % 32;
   const int bh = row / QC;
   const uint8_t* m = map + (int64_t)row * KC;
   const int32_t* off = k_offsets + (int64_t)bh * (KC + 1);
   int2* out = runs + (int64_t)row * max_runs;
-  bool carry = false;
-  int n_start = 0, n_end = 0;
-  for (int base = 0; base <= KC; base += 32) {
-    const int j = base + lane;
-    int o0 = 0;
-    bool act = false;
-    if (j <= KC) o0 = off[j];
-    if (j < KC) act = m[j] != 0 && off[j + 1] > o0;
-    const unsigned bal = __ballot_sync(0xffffffffu, act);
-    const bool prev = lane > 0 ? ((bal >> (lane - 1)) & 1u) : carry;
-    const bool is_start = act && !prev;
-    const bool is_end = (j <= KC) && !act && prev;
-    const unsigned sb = __ballot_sync(0xffffffffu, is_start);
-    const unsigned eb = __ballot_sync(0xffffffffu, is_end);
-    const unsigned lt = (1u << lane) - 1u;
-    if (is_start) { const int r = n_start + __popc(sb & lt); if (r < max_runs) out[r].x = o0; }
-    if (is_end) { const int r = n_end + __popc(eb & lt); if (r < max_runs) out[r].y = o0; }
-    n_start += __popc(sb);
-    n_end += __popc(eb);
-    carry = (bal >> 31) & 1u;
+  const int limit = max_runs - (kEar ? 2 : 1);
+  bool carry = false;                                    // the cluster before this chunk is in a run
+  int n = 0, vbeg = 0;                                   // runs and selected rows so far
+  constexpr int kU = 4;
+  for (int base = 0; base < KC; base += 32 * kU) {       // the loads of kU chunks are in flight together
+    int first[kU], size[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int j = base + u * 32 + lane;
+      first[u] = size[u] = 0;
+      if (j < KC) {
+        first[u] = off[j];
+        size[u] = m[j] != 0 ? off[j + 1] - first[u] : 0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      int incl = size[u];
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, s);
+        if (lane >= s) incl += o;
+      }
+      const bool act = size[u] > 0;
+      const unsigned bal = __ballot_sync(0xffffffffu, act);
+      const unsigned starts = bal & ~((bal << 1) | (carry ? 1u : 0u));
+      if ((starts >> lane) & 1u) {
+        const int r = n + __popc(starts & ((1u << lane) - 1u));
+        if (r < limit) out[r] = make_int2(first[u], vbeg + incl - size[u]);
+      }
+      n += __popc(starts);
+      vbeg += __shfl_sync(0xffffffffu, incl, 31);
+      carry = (bal >> 31) != 0;
+    }
   }
-  const int n = n_start < max_runs - 1 ? n_start : max_runs - 1;
-  __syncwarp();
   if (lane == 0) {
-    int vbeg = 0;
-    for (int r = 0; r < n; ++r) {
-      const int2 se = out[r];
-      out[r] = make_int2(se.x, vbeg);
-      vbeg += se.y - se.x;
+    n = min(n, limit);
+    if (kEar) {
+      out[n++] = make_int2((BH - bh) * S + bh * KC, vbeg);           // the head's centroid rows
+      vbeg += KC;
     }
     out[n] = make_int2(0, vbeg);
     nruns[row] = n;
+    atomicAdd(&head_work[bh], (vbeg + 127) / 128);
   }
 }
 
-// One CTA per head: the query tiles (`tile_rows` rows each) of every non-empty query cluster, in
-// cluster order.  Thread i owns clusters 2i and 2i + 1, so up to 2048 clusters fit one CTA.
-__global__ void __launch_bounds__(1024) build_qtiles_kernel(const int32_t* __restrict__ q_offsets,
-                                                            int4* __restrict__ qtiles, int32_t* __restrict__ nqtiles,
-                                                            int QC, int max_tiles, int tile_rows) {
-  __shared__ int warp_tot[32];
-  const int bh = blockIdx.x, i = threadIdx.x, lane = i % 32, warp = i / 32;
-  const int32_t* off = q_offsets + (int64_t)bh * (QC + 1);
-  int b[3] = {0, 0, 0};
-#pragma unroll
-  for (int u = 0; u < 3; ++u)
-    if (2 * i + u <= QC) b[u] = off[2 * i + u];
-  const int nt0 = 2 * i < QC ? (b[1] - b[0] + tile_rows - 1) / tile_rows : 0;
-  const int nt1 = 2 * i + 1 < QC ? (b[2] - b[1] + tile_rows - 1) / tile_rows : 0;
-  const int nt = nt0 + nt1;
-  int incl = nt;
-#pragma unroll
-  for (int s = 1; s < 32; s <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, incl, s);
-    if (lane >= s) incl += o;
+template <int kRows, bool kSplit, bool kEar>
+__global__ void __launch_bounds__(kListThreads) attn_lists_kernel(
+    const int32_t* __restrict__ q_offsets, int4* __restrict__ qtiles, int32_t* __restrict__ nqtiles, int max_tiles,
+    const uint8_t* __restrict__ map, const int32_t* __restrict__ k_offsets, int2* __restrict__ runs,
+    int32_t* __restrict__ nruns, int32_t* __restrict__ sched, int32_t* __restrict__ head_order, int BH, int S, int QC, int KC,
+    int max_runs) {
+  if ((int)blockIdx.x < BH) {
+    const int bh = blockIdx.x;
+    build_qtiles<kRows, kSplit>(q_offsets + (int64_t)bh * (QC + 1), qtiles + (int64_t)bh * max_tiles, nqtiles + 2 * bh, QC, max_tiles);
+  } else {
+    const int row = (blockIdx.x - BH) * (kListThreads / 32) + threadIdx.x / 32;
+    if (row < BH * QC) build_runs<kEar>(map, k_offsets, runs, nruns, sched + 1, row, BH, S, QC, KC, max_runs);
   }
-  if (lane == 31) warp_tot[warp] = incl;
+  // The last block to finish orders the heads by their selected key tiles (summed over query clusters).
+  __shared__ bool last;
   __syncthreads();
-  if (warp == 0) {
-    int t = warp_tot[lane];
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, t, s);
-      if (lane >= s) t += o;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(sched, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int h = threadIdx.x; h < BH; h += kListThreads) {
+    int rank = h;
+    if (BH <= 1024) {                                    // more heads: any order ends evenly
+      const int mine = __ldcg(sched + 1 + h);
+      rank = 0;
+      for (int g = 0; g < BH; ++g) {
+        const int w = __ldcg(sched + 1 + g);
+        rank += w > mine || (w == mine && g < h);
+      }
     }
-    warp_tot[lane] = t;
+    head_order[rank] = h;
   }
-  __syncthreads();
-  int pos = incl - nt + (warp ? warp_tot[warp - 1] : 0);
-  int4* out = qtiles + (int64_t)bh * max_tiles;
-  if (nt0)
-    for (int r = b[0]; r < b[1]; r += tile_rows, ++pos)
-      if (pos < max_tiles) out[pos] = make_int4(2 * i, r, min(r + tile_rows, b[1]), 0);
-  if (nt1)
-    for (int r = b[1]; r < b[2]; r += tile_rows, ++pos)
-      if (pos < max_tiles) out[pos] = make_int4(2 * i + 1, r, min(r + tile_rows, b[2]), 0);
-  if (i == 1023) nqtiles[bh] = min(warp_tot[31], max_tiles);
 }
 
 cudaError_t launch_block_map(const void* qc, const void* kc, const int32_t* ksizes, uint8_t* map, int64_t BH,
@@ -333,18 +395,17 @@ cudaError_t launch_append_text_blocks(const uint8_t* map, const int32_t* q_off, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_build_runs(const uint8_t* map, const int32_t* k_offsets, int2* runs, int32_t* nruns, int64_t BH,
-                              int64_t QC, int64_t KC, cudaStream_t st) {
-  const int rows = (int)(BH * QC);
-  build_runs_kernel<<<(unsigned)ceil_div(rows, 8), 256, 0, st>>>(map, k_offsets, runs, nruns, (int)QC, (int)KC,
-                                                                 max_runs(KC), rows);
-  count_launches(1);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_build_qtiles(const int32_t* q_offsets, int4* qtiles, int32_t* nqtiles, int64_t BH, int64_t N,
-                                int64_t QC, int tile_rows, cudaStream_t st) {
-  build_qtiles_kernel<<<(unsigned)BH, 1024, 0, st>>>(q_offsets, qtiles, nqtiles, (int)QC, max_qtiles(N, QC), tile_rows);
+// tile_rows: 128 (mma.sync kernel) or 256; split: single tiles in their own list.  ear: with the head's
+// centroid run (256-row tiles only).
+cudaError_t launch_attn_lists(const int32_t* q_offsets, int4* qtiles, int32_t* nqtiles, const uint8_t* map,
+                              const int32_t* k_offsets, int2* runs, int32_t* nruns, int32_t* sched, int32_t* head_order, int64_t BH,
+                              int64_t S, int64_t QC, int64_t KC, int max_runs, int tile_rows, bool split, bool ear, cudaStream_t st) {
+  auto* kernel = tile_rows == 128 ? &attn_lists_kernel<128, false, false>
+                 : ear ? (split ? &attn_lists_kernel<256, true, true> : &attn_lists_kernel<256, false, true>)
+                       : (split ? &attn_lists_kernel<256, true, false> : &attn_lists_kernel<256, false, false>);
+  const int64_t blocks = BH + ceil_div64(BH * QC, kListThreads / 32);
+  kernel<<<(unsigned)blocks, kListThreads, 0, st>>>(q_offsets, qtiles, nqtiles, max_qtiles(S, QC), map, k_offsets, runs, nruns,
+                                                   sched, head_order, (int)BH, (int)S, (int)QC, (int)KC, max_runs);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -31,11 +31,13 @@ struct Workspace {
   int64_t w_hi;          // bf16  [BH, Jpad, 128]
   int64_t w_lo;          // bf16  [BH, Jpad, 128]
   int64_t assign_partial;  // int2 [Jpad/128, BH, N]: best (score bits, j) per column group
+  int64_t sched;         // int32 [1 + BH]: block counter and work per head of attn_lists_kernel; ends where status begins
   int64_t status;        // int32 [4]: word 0 != 0 after a kernel gave up on a bounded wait
   int64_t runs;          // int2  [BH, QC, max_runs]: (first_row, virtual_begin) + sentinel (0, total)
   int64_t nruns;         // int32 [BH, QC]
-  int64_t qtiles;        // int4  [BH, max_qtiles]
-  int64_t nqtiles;       // int32 [BH]
+  int64_t qtiles;        // int4  [BH, max_qtiles]: pair tiles from the front, single tiles in the last QC entries
+  int64_t nqtiles;       // int32 [BH, 2]: pair tiles, single tiles
+  int64_t head_order;    // int32 [BH]: heads by decreasing work
   int64_t total;
 };
 
@@ -43,6 +45,15 @@ __host__ inline int sort_chunks(int64_t N) { return (int)ceil_div64(N, kSortChun
 __host__ inline int pad_clusters(int64_t K) { return (int)align_up(K, 256); }   // W rows, whole 256-row blocks
 __host__ inline int max_runs(int64_t KC) { return (int)(KC / 2 + 2); }   // + one sentinel entry
 __host__ inline int max_qtiles(int64_t N, int64_t QC) { return (int)(ceil_div64(N, kAttnBM) + QC); }
+
+// Query tiles of at most 128 rows go to the kernel of attn_small.cu, unless they are the few remainders of
+// large query clusters.  Attention of 10 x 20,000 tokens with 256 / 160 clusters (78 rows per query cluster):
+// 914 -> 632 us; 12 x 32,760, 100 / 500 (328 rows): 1630 -> 1483; 8 x 59,400, 100 / 800 (594): 2752 -> 2717;
+// 5 x 75,600, 100 / 500 (756): 2129 -> 2157.
+__host__ inline bool single_tile_kernel_wins(int64_t S, int64_t QC) { return S < 640 * QC; }
+// Mean key cluster of at most 100 rows: tiles of too many TMA boxes occur (14 boxes per tile at 65 rows, 9 at
+// 151, where TMA keeps up and the box count per tile is time lost: 2062 -> 2091 us at 5 x 75,600).
+__host__ inline bool short_key_runs(int64_t S, int64_t KC) { return S < 100 * KC; }
 
 __host__ inline Workspace workspace_layout(int64_t BH, int64_t N, int64_t QC, int64_t KC) {
   Workspace w;
@@ -54,12 +65,14 @@ __host__ inline Workspace workspace_layout(int64_t BH, int64_t N, int64_t QC, in
   w.w_hi = take(BH * (int64_t)pad_clusters(Kmax) * kRowBytes);
   w.w_lo = take(BH * (int64_t)pad_clusters(Kmax) * kRowBytes);
   w.assign_partial = take((int64_t)(pad_clusters(Kmax) / 128) * BH * N * 8);   // two column groups per 256 rows
+  w.sched = take((BH + 1) * 4);
   w.status = take(16);
   // sized symmetrically in (QC, KC) so that one workspace serves either side
   w.runs = take(BH * (QC * KC / 2 + 2 * (QC + KC)) * 8);
   w.nruns = take(BH * Kmax * 4);
   w.qtiles = take(BH * (int64_t)max_qtiles(N, Kmax) * 16);
-  w.nqtiles = take(BH * 4);
+  w.nqtiles = take(BH * 8);
+  w.head_order = take(BH * 4);
   w.total = o;
   return w;
 }

@@ -1,0 +1,93 @@
+"""The attention kernels where their tilings can go wrong: query clusters around the 64 / 128 / 256-row tile
+edges, key lists around the 64 / 128-key step edges, runs of single rows (more than 32 per tile), empty
+clusters and empty rows of the map -- against a plain fp32 softmax.
+
+Bound: every weight is rounded to bf16 (2^-9 relative, the weights sum to 1), the output once more
+(2^-9); fp32 sums and ex2.approx are far below that: 2.5 * 2^-9 * max |v|.
+"""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _offsets(sizes, dev):
+    off = torch.zeros(sizes.shape[0], sizes.shape[1] + 1, dtype=torch.int32)
+    off[:, 1:] = sizes.cumsum(1)
+    return off.to(dev)
+
+
+def _reference(q, k, v, m, qs, ks, scale):
+    out = torch.zeros_like(q, dtype=torch.float32)
+    for h in range(q.shape[0]):
+        rows = torch.repeat_interleave(torch.arange(qs.shape[1]), qs[h])
+        cols = torch.repeat_interleave(torch.arange(ks.shape[1]), ks[h])
+        keep = m[h].bool()[rows][:, cols].to(q.device)
+        s = (q[h].float() @ k[h].float().T) * scale
+        p = torch.softmax(s.masked_fill(~keep, float("-inf")), -1).nan_to_num(0.0)
+        out[h] = p @ v[h].float()
+    return out
+
+
+CASES = {
+    # query cluster sizes, key cluster sizes, every n-th key cluster selected (shifted by head and query cluster)
+    "tile-edges": ([1, 64, 65, 128, 129, 192, 193, 256, 257, 385, 0, 2], [64, 1, 63, 128, 0, 65, 127, 900, 300, 24], 2),
+    "single-row-runs": ([40, 0, 128, 33, 250, 500, 300, 6], [1] * 600 + [657], 2),
+    "short-runs": ([31] * 30 + [97] * 9, [3, 5, 8, 1] * 106 + [1], 3),
+    "long-runs": ([700, 900, 1, 650], [1100, 900, 251], 1),
+    "large-clusters": ([700, 900, 651], [1100, 900, 251], 1),
+    "large-clusters-short-runs": ([700, 900, 651], [7, 20, 1, 40] * 33 + [7], 2),
+    "few-keys": ([130, 5, 70], [1, 0, 3, 201], 3),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("ear", [False, True])
+def test_attention_tile_edges(name, ear):
+    from svoo_b200 import ops
+    dev = torch.device("cuda")
+    qsz, ksz, nth = CASES[name]
+    H, S = 3, sum(qsz)
+    assert sum(ksz) == S, (sum(qsz), sum(ksz))
+    gen = torch.Generator().manual_seed(11)
+    qs = torch.stack([torch.tensor(qsz)[torch.randperm(len(qsz), generator=gen)] for _ in range(H)])
+    ks = torch.stack([torch.tensor(ksz)[torch.randperm(len(ksz), generator=gen)] for _ in range(H)])
+    q, k, v = ((3.0 if i < 2 else 1.0) * torch.randn(H, S, 128, generator=gen) for i in range(3))
+    q, k, v = (t.to(dev, torch.bfloat16) for t in (q, k, v))
+    QC, KC = len(qsz), len(ksz)
+    sel = (torch.arange(KC)[None, None] + torch.arange(QC)[None, :, None] + torch.arange(H)[:, None, None]) % nth == 0
+    if not ear and QC > 3:
+        sel[0, 3] = False                                          # a query cluster without keys: zero rows
+    m = sel.to(torch.uint8).to(dev)
+    q_off, k_off = _offsets(qs, dev), _offsets(ks, dev)
+    perm = torch.stack([torch.randperm(S, generator=gen) for _ in range(H)]).to(dev, torch.int32)
+    scale = 128 ** -0.5
+    if not ear:
+        got = ops.sparse_attn(q, k, v, m, q_off, k_off, out_row_idx=perm)
+        assert ops.attention_status(dev, H, S, QC, KC) == 0
+        want = _reference(q, k, v, sel, qs, ks, scale)
+        vmax = v.float().abs().max()
+    else:
+        # centroid j of a pruned cluster is a virtual key with bias log(size + 1e-6)
+        kc, vc = (torch.randn(H, KC, 128, generator=gen).to(dev, torch.bfloat16) for _ in range(2))
+        k_ext = torch.cat([k.reshape(-1, 128), kc.reshape(-1, 128)])
+        v_ext = torch.cat([v.reshape(-1, 128), vc.reshape(-1, 128)])
+        got = ops.sparse_attn_ear(q, k_ext, v_ext, m, q_off, k_off, out_row_idx=perm)
+        assert ops.ear_attention_status(dev, H, S, QC, KC) == 0
+        want = torch.zeros(H, S, 128, device=dev)
+        for h in range(H):
+            rows = torch.repeat_interleave(torch.arange(QC), qs[h])
+            cols = torch.repeat_interleave(torch.arange(KC), ks[h])
+            tok = sel[h][rows][:, cols].to(dev)
+            s = (q[h].float() @ k[h].float().T * scale).masked_fill(~tok, float("-inf"))
+            c = q[h].float() @ kc[h].float().T * scale + torch.log(ks[h].float() + 1e-6).to(dev)
+            c = c.masked_fill(sel[h][rows].to(dev), float("-inf"))
+            p = torch.softmax(torch.cat([s, c], 1), -1)
+            want[h] = p @ torch.cat([v[h], vc[h]]).float()
+        vmax = max(v.float().abs().max(), vc.float().abs().max())
+    idx = perm.long()[..., None].expand(-1, -1, 128)
+    err = (torch.gather(got.float(), 1, idx) - want).abs().max()
+    assert err <= 2.5 * 2.0 ** -9 * vmax, float(err)
+    again = ops.sparse_attn(q, k, v, m, q_off, k_off, out_row_idx=perm) if not ear else \
+        ops.sparse_attn_ear(q, k_ext, v_ext, m, q_off, k_off, out_row_idx=perm)
+    assert torch.equal(again, got)
