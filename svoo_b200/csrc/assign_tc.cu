@@ -41,36 +41,86 @@ struct AsgCfg {
                        ACC_FULL = X_EMPTY + kXStages, ACC_EMPTY = ACC_FULL + 2, NUM = ACC_EMPTY + 2;
 };
 
+// (head, W block, token tile) of consecutive job numbers: the divisions are done once, for the CTA's first
+// job.  (64-bit divisions for every job of every role were most of the epilogue's time.)
 struct AsgJob {
   int bh, jb, t;
+  __device__ __forceinline__ AsgJob(int64_t g, int n_jb, int n_xt) {
+    t = (int)(g % n_xt);
+    const int64_t r = g / n_xt;
+    jb = (int)(r % n_jb);
+    bh = (int)(r / n_jb);
+  }
+  __device__ __forceinline__ void next(int n_jb, int n_xt) {
+    if (++t < n_xt) return;
+    t = 0;
+    if (++jb < n_jb) return;
+    jb = 0;
+    ++bh;
+  }
 };
-__device__ __forceinline__ AsgJob asg_job(int64_t g, int n_jb, int n_xt) {
-  AsgJob j;
-  j.t = (int)(g % n_xt);
-  const int64_t r = g / n_xt;
-  j.jb = (int)(r % n_jb);
-  j.bh = (int)(r / n_jb);
-  return j;
+
+// Running first-argmax of one token's scores.  Compares and selects run on the ALU pipe at half rate, and
+// with three of them per score that pipe, not the tensor pipe, set the kernel's time (ncu: ALU 81 % busy).
+// So the scores go eight at a time: a three-input maximum tree (half an instruction per score), one compare
+// with the best so far, and on success the eight scores are kept (moves, which also run on the FMA pipe);
+// the column inside the kept group is looked up once at the end.  Ties go to the lower column and NaN never
+// wins, as with one strict compare per score in column order.
+struct Best {
+  static constexpr int kG = 8;
+  float best;
+  int first;                                    // first column of the kept group
+  float kept[kG];
+  __device__ __forceinline__ void reset() {
+    best = -INFINITY;
+    first = 0;
+#pragma unroll
+    for (int k = 0; k < kG; ++k) kept[k] = -INFINITY;
+  }
+  __device__ __forceinline__ int column() const {
+    int k1 = 0;
+#pragma unroll
+    for (int k = kG - 1; k >= 0; --k)
+      if (kept[k] == best) k1 = k;
+    return first + k1;
+  }
+};
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
 }
 
-// Running first-argmax over 32 accumulator columns starting at column c0; with kBias the
-// per-column bias (shared memory, indexed like the columns) is added to the score first.
+// 32 accumulator columns starting at column c0 (of jlim valid ones); with kBias the per-column bias
+// (shared memory, indexed like the columns) is added to the score first.
 template <bool kBias>
-__device__ __forceinline__ void argmax32(const uint32_t (&r)[32], int c0, int jlim, const float* bias, float& best,
-                                         int& best_c) {
-  if (c0 + 32 <= jlim) {
+__device__ __forceinline__ void argmax32(uint32_t (&r)[32], int c0, int jlim, const float* bias, Best& b) {
+  if (kBias) {
 #pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      float val = __uint_as_float(r[c]);
-      if (kBias) val += bias[c0 + c];
-      if (val > best) { best = val; best_c = c0 + c; }
+    for (int c = 0; c < 32; c += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(bias + c0 + c);
+      r[c] = __float_as_uint(__uint_as_float(r[c]) + t.x);
+      r[c + 1] = __float_as_uint(__uint_as_float(r[c + 1]) + t.y);
+      r[c + 2] = __float_as_uint(__uint_as_float(r[c + 2]) + t.z);
+      r[c + 3] = __float_as_uint(__uint_as_float(r[c + 3]) + t.w);
     }
-  } else {
+  }
+  if (c0 + 32 > jlim) {                         // the last block's columns past the last cluster
 #pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      float val = __uint_as_float(r[c]);
-      if (kBias) val += bias[c0 + c];
-      if (c0 + c < jlim && val > best) { best = val; best_c = c0 + c; }
+    for (int c = 0; c < 32; ++c)
+      if (c0 + c >= jlim) r[c] = 0xff800000u;
+  }
+#pragma unroll
+  for (int g = 0; g < 32; g += Best::kG) {
+    float x[Best::kG];
+#pragma unroll
+    for (int k = 0; k < Best::kG; ++k) x[k] = __uint_as_float(r[g + k]);
+    const float m = max3(max3(x[0], x[1], x[2]), max3(x[3], x[4], x[5]), fmaxf(x[6], x[7]));
+    if (m > b.best) {
+      b.best = m;
+      b.first = c0 + g;
+#pragma unroll
+      for (int k = 0; k < Best::kG; ++k) b.kept[k] = x[k];
     }
   }
 }
@@ -99,6 +149,8 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
   const int64_t g0 = (int64_t)blockIdx.x * per;
   const int64_t g1 = g0 + per < total ? g0 + per : total;
   if (g0 >= g1) return;
+  const int n_jobs = (int)(g1 - g0);
+  AsgJob job(g0, n_jb, n_xt);
 
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t whi_s = base, wlo_s = base + C::kWBytes, x_s = base + 2 * C::kWBytes;
@@ -128,9 +180,8 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0) {
-      int wq = 0, prev_block = -1, i = 0;
-      for (int64_t g = g0; g < g1; ++g, ++i) {
-        const AsgJob job = asg_job(g, n_jb, n_xt);
+      int wq = 0, prev_block = -1;
+      for (int i = 0; i < n_jobs; ++i, job.next(n_jb, n_xt)) {
         const int block = job.bh * n_jb + job.jb;
         if (block != prev_block) {
           if (!mbar_wait(bar(C::W_EMPTY), (wq & 1) ^ 1, abort_flag)) break;
@@ -158,9 +209,8 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     if (lane == 0) {
-      int wq = 0, prev_block = -1, i = 0;
-      for (int64_t g = g0; g < g1; ++g, ++i) {
-        const AsgJob job = asg_job(g, n_jb, n_xt);
+      int wq = 0, prev_block = -1;
+      for (int i = 0; i < n_jobs; ++i, job.next(n_jb, n_xt)) {
         const int block = job.bh * n_jb + job.jb;
         if (block != prev_block) {
           if (!mbar_wait(bar(C::W_FULL), wq & 1, abort_flag)) break;
@@ -185,12 +235,7 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
         }
         tc_commit(bar(C::X_EMPTY + s));
         tc_commit(bar(C::ACC_FULL + b));
-        bool last_of_block = g + 1 >= g1;
-        if (!last_of_block) {
-          const AsgJob nxt = asg_job(g + 1, n_jb, n_xt);
-          last_of_block = nxt.bh * n_jb + nxt.jb != block;
-        }
-        if (last_of_block) tc_commit(bar(C::W_EMPTY));
+        if (i + 1 == n_jobs || job.t + 1 == n_xt) tc_commit(bar(C::W_EMPTY));    // the block's last job here
       }
     }
   } else if (warp >= 4) {
@@ -200,14 +245,12 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     constexpr int HC = JB / 2;                               // columns per half
     uint32_t ra[32], rb[32];
-    int i = 0;
     bool ok = true;
     // Euclidean mode: the bias of the current W block, one private copy per epilogue warp in the
     // shared memory that the (absent) W_lo operand would occupy
     float* bias_s = reinterpret_cast<float*>(gen_base + C::kWBytes) + (warp - 4) * HC;
     int bias_block = -1;
-    for (int64_t g = g0; g < g1 && ok; ++g, ++i) {
-      const AsgJob job = asg_job(g, n_jb, n_xt);
+    for (int i = 0; i < n_jobs && ok; ++i, job.next(n_jb, n_xt)) {
       const int b = i & 1;
       if (kEuclid && job.bh * n_jb + job.jb != bias_block) {
         bias_block = job.bh * n_jb + job.jb;
@@ -223,8 +266,8 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
       tc_fence_after();
       const uint32_t acc = tmem + lane_addr + b * 256 + half * HC;
       const int jlim = J - job.jb * JB - half * HC;            // valid columns of this half (may be <= 0)
-      float best = -INFINITY;
-      int best_c = 0;
+      Best run;
+      run.reset();
       if (kStack) {
 #pragma unroll
         for (int ch = 0; ch < HC / 32; ++ch) {
@@ -233,7 +276,7 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 32; ++c) ra[c] = __float_as_uint(__uint_as_float(ra[c]) + __uint_as_float(rb[c]));
-          argmax32<false>(ra, ch * 32, jlim, bias_s, best, best_c);
+          argmax32<false>(ra, ch * 32, jlim, bias_s, run);
         }
       } else {
       tmem_ld32_nowait(acc, ra);
@@ -241,10 +284,10 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
 #pragma unroll
       for (int ch = 0; ch < HC / 32; ch += 2) {
         tmem_ld32_nowait(acc + (ch + 1) * 32, rb);
-        argmax32<kEuclid>(ra, ch * 32, jlim, bias_s, best, best_c);
+        argmax32<kEuclid>(ra, ch * 32, jlim, bias_s, run);
         tmem_wait_ld();
         if (ch + 2 < HC / 32) tmem_ld32_nowait(acc + (ch + 2) * 32, ra);
-        argmax32<kEuclid>(rb, (ch + 1) * 32, jlim, bias_s, best, best_c);
+        argmax32<kEuclid>(rb, (ch + 1) * 32, jlim, bias_s, run);
         tmem_wait_ld();
       }
       }
@@ -253,7 +296,7 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
       const int n = job.t * kAsgXT + r_local;
       if (n < N)
         partial[((int64_t)(job.jb * 2 + half) * BH + job.bh) * N + n] =
-            make_int2(__float_as_int(best), job.jb * JB + half * HC + best_c);
+            make_int2(__float_as_int(run.best), job.jb * JB + half * HC + run.column());
     }
   }
   tc_fence_before();
