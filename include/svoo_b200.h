@@ -109,19 +109,10 @@ int svoo_b200_sort_labels(const int32_t* labels, int64_t BH, int64_t N, int64_t 
  * partitioned once at start-up, a plug-in that only gets raw pointers from its host, a
  * loop that must not hit the synchronisation an allocation implies).  This entry point has
  * no counterpart in the reference.  Same inputs, outputs and results as
- * svoo_b200_sort_labels; its scratch is a 4 MiB array built into the library image, which
- * every GPU that loads the library keeps resident until the process exits.
+ * svoo_b200_sort_labels.  It needs no scratch memory, allocates nothing and keeps nothing
+ * between calls, so concurrent calls on one GPU do not disturb one another.
  *   - Limit: BH * ceil(N / 2048) * K <= 1,048,576, otherwise SVOO_ERR_STATIC_SCRATCH is
- *     returned and nothing is launched (40 heads x 75,600 tokens x 500 clusters fits).
- *   - It calls no allocating routine.  The first call made with a given device current
- *     looks up the array's device address; make that first call outside any stream capture.
- *   - All calls on one GPU share the one array.  It holds whatever the previous call left
- *     (the kernels overwrite every entry they later read, so no clearing is needed), and
- *     two calls that run concurrently on the same GPU -- different streams, or different
- *     host threads -- would overwrite each other's histograms: order them.
- *   - The looked-up address is kept for the life of the process.  cudaDeviceReset() destroys the
- *     context it belongs to, so a process that resets a device must not call this entry point
- *     on that device afterwards. */
+ *     returned and nothing is launched (40 heads x 75,600 tokens x 500 clusters fits). */
 int svoo_b200_sort_labels_static(const int32_t* labels, int64_t BH, int64_t N, int64_t K,
                                  int32_t* sorted_idx, int32_t* offsets, void* stream);
 

@@ -5,10 +5,10 @@
 namespace svoo {
 cudaError_t launch_gather_rows(const void*, const int32_t*, void*, int64_t, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_prologue(const void*, const void*, void*, void*, int64_t, int64_t, int64_t, cudaStream_t);
-cudaError_t launch_assign_tc(const void*, const void*, const void*, int32_t*, int2*, int32_t*, int64_t, int64_t, int64_t,
-                             int32_t*, cudaStream_t);
-cudaError_t launch_sort_labels(const int32_t*, int64_t, int64_t, int64_t, int32_t*, int32_t*, int32_t*, int32_t*,
-                               cudaStream_t, bool);
+cudaError_t launch_assign_tc(const void*, const void*, const void*, int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
+int assign_groups(int64_t J);
+cudaError_t launch_assign_reduce(const int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
+cudaError_t launch_sort_labels(const int2*, int, int32_t*, int64_t, int64_t, int64_t, int32_t*, int32_t*, int32_t*, cudaStream_t);
 cudaError_t launch_centroid_update(const void*, const int32_t*, const int32_t*, const void*, void*, int32_t*, float*,
                                    int64_t, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_offsets_from_sizes(const int32_t*, int32_t*, int64_t, int64_t, cudaStream_t);
@@ -29,8 +29,7 @@ cudaError_t launch_ear_scores(const void*, const void*, const void*, const int32
                               cudaStream_t);
 cudaError_t launch_ear_select(const float*, const float*, const int32_t*, const int32_t*, uint8_t*, int64_t, int64_t, int64_t,
                               float, const int32_t*, const int32_t*, cudaStream_t);
-cudaError_t launch_euclid_assign_tc(const void*, const void*, float*, int32_t*, int2*, int32_t*, int64_t, int64_t, int64_t,
-                                    int32_t*, cudaStream_t);
+cudaError_t launch_euclid_assign_tc(const void*, const void*, float*, int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_append_text_blocks(const uint8_t*, const int32_t*, const int32_t*, const int32_t*, const int32_t*,
                                       uint8_t*, int32_t*, int32_t*, int32_t*, int32_t*, int64_t, int64_t, int64_t, int64_t,
                                       int64_t, int64_t, cudaStream_t);
@@ -127,9 +126,10 @@ int svoo_b200_cocluster_assign(const void* x, const void* form_centroids, const 
   SVOO_CUDA(launch_prologue(own_centroids, form_centroids, ws_at<void>(workspace, w.w_hi),
                             ws_at<void>(workspace, w.w_lo), BH, J, K, st));
   SVOO_CUDA(cudaMemsetAsync(ws_at<int32_t>(workspace, w.status) + 1, 0, 4, st));
-  SVOO_CUDA(launch_assign_tc(x, ws_at<void>(workspace, w.w_hi), ws_at<void>(workspace, w.w_lo), labels,
-                             ws_at<int2>(workspace, w.assign_partial), ws_at<int32_t>(workspace, w.status) + 1, BH, N, J, nullptr,
-                             st));
+  int2* partial = ws_at<int2>(workspace, w.assign_partial);
+  SVOO_CUDA(launch_assign_tc(x, ws_at<void>(workspace, w.w_hi), ws_at<void>(workspace, w.w_lo), partial,
+                             ws_at<int32_t>(workspace, w.status) + 1, BH, N, J, st));
+  SVOO_CUDA(launch_assign_reduce(partial, labels, BH, N, J, st));
   return SVOO_OK;
 }
 
@@ -144,8 +144,9 @@ int svoo_b200_euclid_assign(const void* x, const void* centroids, int64_t BH, in
   cudaStream_t st = (cudaStream_t)stream;
   int32_t* status = ws_at<int32_t>(workspace, w.status) + 1;
   SVOO_CUDA(cudaMemsetAsync(status, 0, 4, st));
-  SVOO_CUDA(launch_euclid_assign_tc(x, centroids, ws_at<float>(workspace, w.w_hi), labels,
-                                    ws_at<int2>(workspace, w.assign_partial), status, BH, N, K, nullptr, st));
+  int2* partial = ws_at<int2>(workspace, w.assign_partial);
+  SVOO_CUDA(launch_euclid_assign_tc(x, centroids, ws_at<float>(workspace, w.w_hi), partial, status, BH, N, K, st));
+  SVOO_CUDA(launch_assign_reduce(partial, labels, BH, N, K, st));
   return SVOO_OK;
 }
 
@@ -156,8 +157,8 @@ int svoo_b200_sort_labels(const int32_t* labels, int64_t BH, int64_t N, int64_t 
   SVOO_TRY(check_clusters(K));
   const Workspace w = workspace_layout(BH, N, K, K);
   if (workspace_bytes < w.total) return SVOO_ERR_WORKSPACE;
-  SVOO_CUDA(launch_sort_labels(labels, BH, N, K, sorted_idx, offsets, nullptr, ws_at<int32_t>(workspace, w.chunk_hist),
-                               (cudaStream_t)stream, false));
+  SVOO_CUDA(launch_sort_labels(nullptr, 0, const_cast<int32_t*>(labels), BH, N, K, sorted_idx, offsets, nullptr,
+                               (cudaStream_t)stream));
   return SVOO_OK;
 }
 
@@ -196,7 +197,6 @@ int svoo_b200_cocluster(const void* q, const void* k, const int32_t* q_init_idx,
   cudaStream_t st = (cudaStream_t)stream;
   void* w_hi = ws_at<void>(workspace, w.w_hi);
   void* w_lo = ws_at<void>(workspace, w.w_lo);
-  int32_t* hist = ws_at<int32_t>(workspace, w.chunk_hist);
   float* partial = ws_at<float>(workspace, w.partial);
   int2* apart = ws_at<int2>(workspace, w.assign_partial);
   int32_t* status = ws_at<int32_t>(workspace, w.status) + 1;       // word 1: assignment kernel
@@ -209,13 +209,13 @@ int svoo_b200_cocluster(const void* q, const void* k, const int32_t* q_init_idx,
   for (int it = 0; it < iters; ++it) {
     // keys: profile over the query centroids
     SVOO_CUDA(launch_prologue(kcentroids, qcentroids, w_hi, w_lo, BH, KC, QC, st));
-    SVOO_CUDA(launch_assign_tc(k, w_hi, w_lo, klabels, apart, status, BH, N, KC, hist, st));
-    SVOO_CUDA(launch_sort_labels(klabels, BH, N, KC, k_sorted_idx, k_offsets, nullptr, hist, st, true));
+    SVOO_CUDA(launch_assign_tc(k, w_hi, w_lo, apart, status, BH, N, KC, st));
+    SVOO_CUDA(launch_sort_labels(apart, assign_groups(KC), klabels, BH, N, KC, k_sorted_idx, k_offsets, nullptr, st));
     SVOO_CUDA(launch_centroid_update(k, k_sorted_idx, k_offsets, kcentroids, kcentroids, ksizes, partial, BH, N, KC, st));
     // queries: profile over the just-updated key centroids
     SVOO_CUDA(launch_prologue(qcentroids, kcentroids, w_hi, w_lo, BH, QC, KC, st));
-    SVOO_CUDA(launch_assign_tc(q, w_hi, w_lo, qlabels, apart, status, BH, N, QC, hist, st));
-    SVOO_CUDA(launch_sort_labels(qlabels, BH, N, QC, q_sorted_idx, q_offsets, nullptr, hist, st, true));
+    SVOO_CUDA(launch_assign_tc(q, w_hi, w_lo, apart, status, BH, N, QC, st));
+    SVOO_CUDA(launch_sort_labels(apart, assign_groups(QC), qlabels, BH, N, QC, q_sorted_idx, q_offsets, nullptr, st));
     SVOO_CUDA(launch_centroid_update(q, q_sorted_idx, q_offsets, qcentroids, qcentroids, qsizes, partial, BH, N, QC, st));
   }
   return SVOO_OK;

@@ -16,7 +16,8 @@
 //               and one half of the accumulator columns: running first-argmax, one (score, j)
 //               pair per token and column group written to scratch
 //
-// A small second kernel reduces the per-block pairs to labels (lower block wins ties).
+// The label sort (cluster.cu), or a small kernel when only labels are wanted, reduces the pairs to labels
+// (lower column group wins ties).
 // Every mbarrier wait is bounded; on expiry the CTA sets the status word and leaves.
 #include "tc_common.cuh"
 
@@ -323,38 +324,6 @@ __global__ void __launch_bounds__(256) assign_reduce_kernel(const int2* __restri
   labels[i] = b.y;
 }
 
-// The same reduction fused with the first pass of the label sort: one CTA per (2048-token chunk,
-// head) also leaves the chunk's label histogram, which saves a kernel and a second read of the labels.
-__global__ void __launch_bounds__(256) assign_reduce_hist_kernel(const int2* __restrict__ partial,
-                                                                 int32_t* __restrict__ labels,
-                                                                 int32_t* __restrict__ chunk_hist, int BH, int N, int K,
-                                                                 int groups, int nchunks) {
-  __shared__ int hist[SVOO_MAX_CLUSTERS];
-  pdl_trigger();
-  const int bh = blockIdx.y, chunk = blockIdx.x;
-  for (int k = threadIdx.x; k < K; k += 256) hist[k] = 0;
-  __syncthreads();
-  pdl_wait();
-  const int64_t BHN = (int64_t)BH * N;
-  const int base = chunk * kSortChunk;
-  for (int t = threadIdx.x; t < kSortChunk; t += 256) {
-    const int n = base + t;
-    if (n < N) {
-      const int64_t i = (int64_t)bh * N + n;
-      int2 b = partial[i];
-      for (int g = 1; g < groups; ++g) {
-        const int2 c = partial[(int64_t)g * BHN + i];
-        if (__int_as_float(c.x) > __int_as_float(b.x)) b = c;
-      }
-      labels[i] = b.y;
-      if (b.y >= 0 && b.y < K) atomicAdd(&hist[b.y], 1);
-    }
-  }
-  __syncthreads();
-  int32_t* out = chunk_hist + ((int64_t)bh * nchunks + chunk) * K;
-  for (int k = threadIdx.x; k < K; k += 256) out[k] = hist[k];
-}
-
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -406,29 +375,22 @@ static cudaError_t launch_assign_tc_jb(const void* x, const void* w_hi, const vo
                     partial, (int)BH, (int)N, (int)J, w_head_rows, bias, status);
 }
 
-static cudaError_t launch_assign_reduce(const int2* partial, int32_t* labels, int64_t BH, int64_t N, int64_t J, int jb,
-                                        int32_t* chunk_hist, cudaStream_t st) {
-  const int groups = 2 * (int)ceil_div64(J, jb);
-  if (chunk_hist) {
-    const int nchunks = sort_chunks(N);
-    count_launches(2);
-    return launch_pdl(tc::assign_reduce_hist_kernel, dim3((unsigned)nchunks, (unsigned)BH), dim3(256), 0, st,
-                      (const int2*)partial, labels, chunk_hist, (int)BH, (int)N, (int)J, groups, nchunks);
-  }
-  count_launches(2);
+// Column groups per token in `partial`: two per W block.
+int assign_groups(int64_t J) { return 2 * (int)ceil_div64(J, J <= 128 ? 128 : 256); }
+
+cudaError_t launch_assign_reduce(const int2* partial, int32_t* labels, int64_t BH, int64_t N, int64_t J, cudaStream_t st) {
+  count_launches(1);
   return launch_pdl(tc::assign_reduce_kernel, dim3((unsigned)ceil_div64(BH * N, 256)), dim3(256), 0, st, (const int2*)partial,
-                    labels, BH * N, groups);
+                    labels, BH * N, assign_groups(J));
 }
 
-// chunk_hist != nullptr: also write the per-chunk label histograms of the sort (its first pass).
-cudaError_t launch_assign_tc(const void* x, const void* w_hi, const void* w_lo, int32_t* labels, int2* partial,
-                             int32_t* status, int64_t BH, int64_t N, int64_t J, int32_t* chunk_hist, cudaStream_t st) {
+// Leaves the winners of the column groups in `partial`; the label sort or launch_assign_reduce reads them.
+cudaError_t launch_assign_tc(const void* x, const void* w_hi, const void* w_lo, int2* partial, int32_t* status, int64_t BH,
+                             int64_t N, int64_t J, cudaStream_t st) {
   const int Jpad = pad_clusters(J);
-  const int jb = J <= 128 ? 128 : 256;
-  cudaError_t e = jb == 128 ? launch_assign_tc_jb<128, false>(x, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st)
-                            : launch_assign_tc_jb<256, false>(x, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st);
-  if (e != cudaSuccess) return e;
-  return launch_assign_reduce(partial, labels, BH, N, J, jb, chunk_hist, st);
+  count_launches(1);
+  return J <= 128 ? launch_assign_tc_jb<128, false>(x, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st)
+                  : launch_assign_tc_jb<256, false>(x, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st);
 }
 
 // bias[bh, j] = -sum_d bf16(c_d * c_d) / 2: the centroid term of the squared distance with the
@@ -453,20 +415,16 @@ __global__ void __launch_bounds__(256) euclid_bias_kernel(const bf16* __restrict
   if (lane == 0) bias[row] = -0.5f * s;
 }
 
-// labels[bh, n] = first argmin_j |x_n - c_j|^2 (svoo/co_clustering.py:335-416): the assignment GEMM with
+// Winners of first argmin_j |x_n - c_j|^2 (svoo/co_clustering.py:335-416): the assignment GEMM with
 // the centroids themselves as the stationary operand and -|c_j|^2 / 2 added in the epilogue.
-cudaError_t launch_euclid_assign_tc(const void* x, const void* centroids, float* bias, int32_t* labels, int2* partial,
-                                    int32_t* status, int64_t BH, int64_t N, int64_t K, int32_t* chunk_hist, cudaStream_t st) {
-  cudaError_t eb = launch_pdl(euclid_bias_kernel, dim3((unsigned)ceil_div64(BH * K, 16)), dim3(256), 0, st,
-                              (const bf16*)centroids, bias, BH * K);
-  if (eb != cudaSuccess) return eb;
-  count_launches(1);
-  const int jb = K <= 128 ? 128 : 256;
-  cudaError_t e = jb == 128
-      ? launch_assign_tc_jb<128, true>(x, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st)
-      : launch_assign_tc_jb<256, true>(x, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st);
+cudaError_t launch_euclid_assign_tc(const void* x, const void* centroids, float* bias, int2* partial, int32_t* status,
+                                    int64_t BH, int64_t N, int64_t K, cudaStream_t st) {
+  cudaError_t e = launch_pdl(euclid_bias_kernel, dim3((unsigned)ceil_div64(BH * K, 16)), dim3(256), 0, st,
+                             (const bf16*)centroids, bias, BH * K);
   if (e != cudaSuccess) return e;
-  return launch_assign_reduce(partial, labels, BH, N, K, jb, chunk_hist, st);
+  count_launches(2);
+  return K <= 128 ? launch_assign_tc_jb<128, true>(x, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st)
+                  : launch_assign_tc_jb<256, true>(x, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st);
 }
 
 }  // namespace svoo

@@ -208,52 +208,131 @@ __global__ void __launch_bounds__(256) profile_prologue_kernel(
 }
 
 // ---------------------------------------------------------------------------------------
-// Stable counting sort of labels (three kernels).
+// Stable counting sort of the labels of a head, in one launch: a cluster of up to 16 CTAs per head.
+// Every warp owns a contiguous range of tokens and counts its labels in a histogram of its own.  The CTAs exchange their
+// totals through distributed shared memory, every CTA scans the head's totals, and a second walk over the
+// same tokens writes them to their places.
+// kGroups > 0: the labels are first reduced from the assignment kernel's per-column-group winners
+// (lower group wins ties) and written out on the way.
+//
+// As separate histogram, scan and scatter kernels this was three of the seven launches of a clustering
+// phase, each of them a chain of dependent loads.  Mean of both sides, 100 / 500 clusters: 12 x 32,760 tokens
+// 19.2 -> 11.3 us, 5 x 75,600 20.6 -> 15.2, 40 x 75,600 55 -> 47; 2 x 4,096, 32 / 128: 12.4 -> 6.4.  What is left
+// is shared-memory work: an atomic per token in the first walk, a match and two accesses in the second.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) label_hist_kernel(const int32_t* __restrict__ labels,
-                                                         int32_t* __restrict__ chunk_hist, int N, int K, int nchunks) {
-  __shared__ int hist[SVOO_MAX_CLUSTERS];
-  pdl_trigger();
-  const int bh = blockIdx.y, chunk = blockIdx.x;
-  for (int k = threadIdx.x; k < K; k += 256) hist[k] = 0;
-  __syncthreads();
-  pdl_wait();
-  const int base = chunk * kSortChunk;
-  for (int i = threadIdx.x; i < kSortChunk; i += 256) {
-    const int n = base + i;
-    if (n < N) {
-      const int l = labels[(int64_t)bh * N + n];
-      if (l >= 0 && l < K) atomicAdd(&hist[l], 1);
-    }
-  }
-  __syncthreads();
-  int32_t* out = chunk_hist + ((int64_t)bh * nchunks + chunk) * K;
-  for (int k = threadIdx.x; k < K; k += 256) out[k] = hist[k];
+constexpr int kSortWarps = 16;
+constexpr int kSortThreads = 32 * kSortWarps;
+constexpr int kSortCtasPerSm = 3;
+constexpr int kSortMaxCluster = 16;
+inline size_t sort_smem_bytes(int64_t K) { return (size_t)(kSortWarps + 2) * K * 4; }          // 72 KB at 1024 clusters
+
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ int ld_cluster(uint32_t addr, uint32_t rank) {
+  int v;
+  asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.s32 %0, [a];\n\t}\n"
+               : "=r"(v) : "r"(addr), "r"(rank) : "memory");
+  return v;
 }
 
-// One CTA per head: per-cluster exclusive prefix over chunks (in place), totals, offsets.
-__global__ void __launch_bounds__(1024) label_scan_kernel(int32_t* __restrict__ chunk_hist, int32_t* __restrict__ offsets,
-                                                          int32_t* __restrict__ sizes, int K, int nchunks) {
-  __shared__ int warp_tot[32];
+template <int kGroups>
+__global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kernel(
+    const int2* __restrict__ partial, int32_t* labels, int32_t* __restrict__ sorted_idx, int32_t* __restrict__ offsets,
+    int32_t* __restrict__ sizes, int BH, int N, int K) {
+  extern __shared__ int sort_sm[];
+  int* wh = sort_sm;                                     // [16][K] counts, then positions, per warp
+  int* tot = wh + kSortWarps * K;                        // [K] this CTA's totals
+  int* add = tot + K;                                    // [K] first position of this CTA's tokens of a label
+  __shared__ int warp_tot[kSortWarps];
   pdl_trigger();
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int rank = (int)cluster_rank(), ctas = (int)cluster_size();
+  const int bh = blockIdx.x / ctas;
+  for (int i = tid; i < kSortWarps * K; i += kSortThreads) wh[i] = 0;
+  // ranges are whole groups of 32 tokens
+  const int per_cta = (int)ceil_div64(ceil_div64(N, ctas), 32) * 32;
+  const int c0 = min(rank * per_cta, N), c1 = min(c0 + per_cta, N);
+  const int per_warp = ceil_div(ceil_div(c1 - c0, kSortWarps), 32) * 32;
+  const int w0 = min(c0 + warp * per_warp, c1), w1 = min(w0 + per_warp, c1);
+  int* mine = wh + warp * K;
+  int32_t* lb = labels + (int64_t)bh * N;
+  __syncthreads();
   pdl_wait();
-  const int bh = blockIdx.x, k = threadIdx.x, lane = k % 32, warp = k / 32;
-  int total = 0;
-  if (k < K) {
-    int32_t* col = chunk_hist + (int64_t)bh * nchunks * K + k;
-    for (int c0 = 0; c0 < nchunks; c0 += 8) {          // 8 independent loads in flight, then the stores
-      int v[8];
+
+  // ---- walk 1: labels and the warp's counts; the loads of kU steps are in flight together
+  constexpr int kU = kGroups > 2 ? (kGroups > 4 ? 1 : 2) : 4;
+  for (int s = w0; s < w1; s += 32 * kU) {
+    int l[kU];
+    if constexpr (kGroups == 0) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = (c0 + u < nchunks) ? col[(int64_t)(c0 + u) * K] : 0;
+      for (int u = 0; u < kU; ++u) {
+        const int n = s + u * 32 + lane;
+        l[u] = n < w1 ? lb[n] : -1;
+      }
+    } else {
+      int2 c[kU][kGroups];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (c0 + u < nchunks) col[(int64_t)(c0 + u) * K] = total;
-        total += v[u];
+      for (int u = 0; u < kU; ++u) {
+        const int n = min(s + u * 32 + lane, w1 - 1);
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) c[u][g] = partial[((int64_t)g * BH + bh) * N + n];
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int n = s + u * 32 + lane;
+        int2 best = c[u][0];
+#pragma unroll
+        for (int g = 1; g < kGroups; ++g)
+          if (__int_as_float(c[u][g].x) > __int_as_float(best.x)) best = c[u][g];
+        l[u] = n < w1 ? best.y : -1;
+        if (n < w1) lb[n] = best.y;
       }
     }
-    if (sizes) sizes[(int64_t)bh * K + k] = total;
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (l[u] >= 0 && l[u] < K) atomicAdd(&mine[l[u]], 1);
+    }
   }
-  int incl = total;
+  __syncthreads();
+  for (int k = tid; k < K; k += kSortThreads) {
+    int run = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+      const int t = wh[w * K + k];
+      wh[w * K + k] = run;
+      run += t;
+    }
+    tot[k] = run;
+  }
+  cluster_arrive();
+  cluster_wait();
+
+  // ---- totals of the head and of the CTAs before this one; exclusive scan over the labels
+  constexpr int kPer = (SVOO_MAX_CLUSTERS + kSortThreads - 1) / kSortThreads;
+  const int per = ceil_div(K, kSortThreads);             // labels per thread
+  int all[kPer], before[kPer], sum = 0;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = tid * per + u;
+    all[u] = before[u] = 0;
+    if (u < per && k < K)
+      for (int r0 = 0; r0 < ctas; r0 += 8) {             // eight remote reads in flight
+        int v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[r] = ld_cluster(smem_u32(tot + k), min(r0 + r, ctas - 1));
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if (r0 + r >= ctas) v[r] = 0;
+          if (r0 + r < rank) before[u] += v[r];
+          all[u] += v[r];
+        }
+      }
+    sum += all[u];
+  }
+  cluster_arrive();                                      // this CTA has read the others' totals (waited for at the end)
+  int incl = sum;
 #pragma unroll
   for (int s = 1; s < 32; s <<= 1) {
     const int o = __shfl_up_sync(0xffffffffu, incl, s);
@@ -261,73 +340,53 @@ __global__ void __launch_bounds__(1024) label_scan_kernel(int32_t* __restrict__ 
   }
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
-  if (warp == 0) {
-    int v = warp_tot[lane];
+  int excl = incl - sum, total = 0;
 #pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, v, s);
-      if (lane >= s) v += o;
-    }
-    warp_tot[lane] = v;
+  for (int w = 0; w < kSortWarps; ++w) {
+    if (w < warp) excl += warp_tot[w];
+    total += warp_tot[w];
   }
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = tid * per + u;
+    if (u < per && k < K) {
+      add[k] = excl + before[u];
+      if (rank == 0) {
+        offsets[(int64_t)bh * (K + 1) + k] = excl;
+        if (sizes) sizes[(int64_t)bh * K + k] = all[u];
+      }
+    }
+    excl += all[u];
+  }
+  if (rank == 0 && tid == 0) offsets[(int64_t)bh * (K + 1) + K] = total;
   __syncthreads();
-  const int excl = incl - total + (warp ? warp_tot[warp - 1] : 0);
-  if (k < K) offsets[(int64_t)bh * (K + 1) + k] = excl;
-  if (k == K - 1) offsets[(int64_t)bh * (K + 1) + K] = excl + total;
-}
 
-__global__ void __launch_bounds__(256) label_scatter_kernel(const int32_t* __restrict__ labels,
-                                                            const int32_t* __restrict__ chunk_base,
-                                                            const int32_t* __restrict__ offsets,
-                                                            int32_t* __restrict__ sorted_idx, int N, int K, int nchunks) {
-  extern __shared__ int wh[];          // [8][K] per-warp histogram, then per-warp running position
-  pdl_trigger();
-  const int bh = blockIdx.y, chunk = blockIdx.x;
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  for (int i = tid; i < 8 * K; i += 256) wh[i] = 0;
-  __syncthreads();
-  pdl_wait();
-  const int wbase = chunk * kSortChunk + warp * (kSortChunk / 8);
-  const int32_t* lb = labels + (int64_t)bh * N;
-  int mine[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    const int n = wbase + s * 32 + lane;
-    int l = (n < N) ? lb[n] : -1;
-    if (l >= K) l = -1;
-    mine[s] = l;
-    if (l >= 0) atomicAdd(&wh[warp * K + l], 1);
-  }
-  __syncthreads();
-  const int32_t* cb = chunk_base + ((int64_t)bh * nchunks + chunk) * K;
-  const int32_t* ob = offsets + (int64_t)bh * (K + 1);
-  for (int k = tid; k < K; k += 256) {
-    int run = ob[k] + cb[k];
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      const int t = wh[w * K + k];
-      wh[w * K + k] = run;
-      run += t;
-    }
-  }
-  __syncthreads();
+  // ---- walk 2: the warp's tokens to their places, in order
   int32_t* out = sorted_idx + (int64_t)bh * N;
+  for (int s = w0; s < w1; s += 32 * 4) {
+    int l[4];
 #pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    const int l = mine[s];
-    const unsigned key = (l >= 0) ? (unsigned)l : (unsigned)(SVOO_MAX_CLUSTERS + lane);
-    const unsigned grp = __match_any_sync(0xffffffffu, key);
-    const int rank = __popc(grp & ((1u << lane) - 1u));
-    int base = 0;
-    if (l >= 0) base = wh[warp * K + l];
-    __syncwarp();
-    if (l >= 0 && rank == 0) wh[warp * K + l] = base + __popc(grp);
-    __syncwarp();
-    if (l >= 0) {
-      const int pos = base + rank;
-      if (pos < N) out[pos] = wbase + s * 32 + lane;
+    for (int u = 0; u < 4; ++u) {
+      const int n = s + u * 32 + lane;
+      l[u] = n < w1 ? lb[n] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool ok = l[u] >= 0 && l[u] < K;
+      const unsigned grp = __match_any_sync(0xffffffffu, ok ? l[u] : K + lane);
+      const int pos_in_grp = __popc(grp & ((1u << lane) - 1u));
+      int base = 0;
+      if (ok) base = mine[l[u]];
+      __syncwarp();
+      if (ok && pos_in_grp == 0) mine[l[u]] = base + __popc(grp);
+      __syncwarp();
+      if (ok) {
+        const int pos = add[l[u]] + base + pos_in_grp;
+        if (pos < N) out[pos] = s + u * 32 + lane;
+      }
     }
   }
+  cluster_wait();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -480,21 +539,46 @@ cudaError_t launch_prologue(const void* own, const void* form, void* w_hi, void*
                     (bf16*)w_lo, (int)J, (int)K, Jpad);
 }
 
-// hist_done: chunk_hist already holds the per-chunk label histograms (written by the assignment's
-// reduction), so the first pass is skipped.
-cudaError_t launch_sort_labels(const int32_t* labels, int64_t BH, int64_t N, int64_t K, int32_t* sorted_idx,
-                               int32_t* offsets, int32_t* sizes, int32_t* chunk_hist, cudaStream_t st, bool hist_done) {
-  const int nchunks = sort_chunks(N);
-  // label_scatter_kernel uses 8 * K * 4 <= 32 KB of dynamic shared memory: inside the default limit
-  dim3 grid((unsigned)nchunks, (unsigned)BH);
-  cudaError_t e = cudaSuccess;
-  if (!hist_done) e = launch_pdl(label_hist_kernel, grid, dim3(256), 0, st, labels, chunk_hist, (int)N, (int)K, nchunks);
+// groups > 0: `labels` are first reduced from that many column groups of `partial` (see assign_tc.cu).
+cudaError_t launch_sort_labels(const int2* partial, int groups, int32_t* labels, int64_t BH, int64_t N, int64_t K,
+                               int32_t* sorted_idx, int32_t* offsets, int32_t* sizes, cudaStream_t st) {
+  void (*kernel)(const int2*, int32_t*, int32_t*, int32_t*, int32_t*, int, int, int) = nullptr;
+  switch (groups) {                                      // two per 256 (at most 128 clusters: 128) W rows
+    case 0: kernel = sort_labels_kernel<0>; break;
+    case 2: kernel = sort_labels_kernel<2>; break;
+    case 4: kernel = sort_labels_kernel<4>; break;
+    case 6: kernel = sort_labels_kernel<6>; break;
+    case 8: kernel = sort_labels_kernel<8>; break;
+    default: return cudaErrorInvalidValue;
+  }
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem_bytes(SVOO_MAX_CLUSTERS));
   if (e != cudaSuccess) return e;
-  e = launch_pdl(label_scan_kernel, dim3((unsigned)BH), dim3(1024), 0, st, chunk_hist, offsets, sizes, (int)K, nchunks);
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  count_launches(hist_done ? 2 : 3);
-  return launch_pdl(label_scatter_kernel, grid, dim3(256), (size_t)(8 * K * 4), st, labels, (const int32_t*)chunk_hist,
-                    (const int32_t*)offsets, sorted_idx, (int)N, (int)K, nchunks);
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // As many CTAs per head as surely fit the chip at once (a cluster stays inside one GPC, so the last quarter of
+  // the slots is not counted on), of at least 512 tokens and K (a CTA clears and scans 16 K counters).
+  // 24 heads x 8,505 tokens, 1024 clusters: 34 us with 16 CTAs per head, 16 us with 4.
+  const int64_t slots = (int64_t)sms * kSortCtasPerSm * 3 / 4, min_tokens = K > 512 ? K : 512;
+  int ctas = 1;
+  while (ctas < kSortMaxCluster && BH * ctas * 2 <= slots && N >= ctas * 2 * min_tokens) ctas *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(BH * ctas));
+  cfg.blockDim = dim3(kSortThreads);
+  cfg.dynamicSmemBytes = sort_smem_bytes(K);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)ctas;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  count_launches(1);
+  return cudaLaunchKernelEx(&cfg, kernel, partial, labels, sorted_idx, offsets, sizes, (int)BH, (int)N, (int)K);
 }
 
 cudaError_t launch_centroid_update(const void* x, const int32_t* sorted_idx, const int32_t* offsets,
@@ -524,50 +608,20 @@ cudaError_t launch_offsets_from_sizes(const int32_t* sizes, int32_t* offsets, in
 }  // namespace svoo
 
 // ---------------------------------------------------------------------------------------
-// svoo_b200_sort_labels_static: the label sort for callers that cannot hand over a workspace.
-//
-// Some hosts of this library are not allowed to allocate device memory at the point where
-// they call it: a serving process whose HBM is carved up once at start-up, a plug-in that
-// only ever receives raw pointers from its host framework and has no allocator of its own,
-// or a latency-critical loop that must not risk the implicit device synchronisation of an
-// allocation.  For them the per-chunk histogram scratch of the sort lives in the array
-// below instead of a caller-provided workspace.  The price is a fixed 4 MiB of device
-// memory on every GPU that loads the library, held until the process exits, and a size
-// limit: BH * ceil(N / 2048) * K must not exceed kStaticSortInts.
-//
-// `g_static_sort_scratch` names the array for device code.  In host code the same name is
-// only a stand-in symbol, not a device address, so the launcher asks the runtime for the
-// real address once per device (cudaGetSymbolAddress, with that device current) and
-// passes that pointer to the kernels.
+// svoo_b200_sort_labels_static: the label sort for callers that cannot hand over a workspace (device memory
+// carved up once at start-up, a plug-in without an allocator, a loop that must not meet the implicit
+// synchronisation of an allocation).  The sort keeps its counts in shared memory, so it needs no scratch at
+// all; the size limit of the entry point (it once had a fixed scratch array) is part of its interface.
 // ---------------------------------------------------------------------------------------
-namespace svoo {
-constexpr int64_t kStaticSortInts = 1 << 20;                       // 4 MiB of int32
-constexpr int kMaxDevices = 64;
-static __device__ __align__(256) int32_t g_static_sort_scratch[kStaticSortInts];
-}  // namespace svoo
-
 extern "C" int svoo_b200_sort_labels_static(const int32_t* labels, int64_t BH, int64_t N, int64_t K,
                                             int32_t* sorted_idx, int32_t* offsets, void* stream) {
   using namespace svoo;
+  constexpr int64_t kMaxCounts = 1 << 20, kCountChunk = 2048;
   if (!labels || !sorted_idx || !offsets) return SVOO_ERR_NULL;
   if (BH < 1 || BH > 65535 || N < 1 || N > (1 << 24) || K < 1 || BH * N > (int64_t)INT32_MAX) return SVOO_ERR_SHAPE;
   if (K > SVOO_MAX_CLUSTERS) return SVOO_ERR_CLUSTERS;
-  if (BH * (int64_t)sort_chunks(N) * K > kStaticSortInts) return SVOO_ERR_STATIC_SCRATCH;
-  // Address of the array on the current device, looked up on the first call made with that
-  // device current.  Two host threads racing here would store the same value.
-  static int32_t* scratch_of_device[kMaxDevices] = {};
-  int dev = -1;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return (int)e;
-  if (dev < 0 || dev >= kMaxDevices) return SVOO_ERR_SHAPE;
-  int32_t* scratch = scratch_of_device[dev];
-  if (!scratch) {
-    e = cudaGetSymbolAddress((void**)&scratch, g_static_sort_scratch);
-    if (e != cudaSuccess) return (int)e;
-    scratch_of_device[dev] = scratch;
-  }
-  // Nothing in the array has to start at zero: label_hist_kernel writes every
-  // [head, chunk, cluster] entry that the scan and scatter kernels read afterwards.
-  e = launch_sort_labels(labels, BH, N, K, sorted_idx, offsets, nullptr, scratch, (cudaStream_t)stream, false);
+  if (BH * ceil_div64(N, kCountChunk) * K > kMaxCounts) return SVOO_ERR_STATIC_SCRATCH;
+  cudaError_t e = launch_sort_labels(nullptr, 0, const_cast<int32_t*>(labels), BH, N, K, sorted_idx, offsets, nullptr,
+                                     (cudaStream_t)stream);
   return e == cudaSuccess ? SVOO_OK : (int)e;
 }

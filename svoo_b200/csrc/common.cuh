@@ -21,12 +21,10 @@ __host__ __device__ inline int64_t align_up(int64_t a, int64_t b) { return (a + 
 // ---------------------------------------------------------------------------------------
 // Workspace layout shared by the host entry points.  All offsets are multiples of 256 B.
 // ---------------------------------------------------------------------------------------
-constexpr int kSortChunk = 2048;         // tokens per CTA in the counting sort
 constexpr int kCentroidSlabs = 8;        // partial sums per cluster in the centroid update
 constexpr int kAttnBM = 128;             // query rows per attention tile
 
 struct Workspace {
-  int64_t chunk_hist;    // int32 [BH, nchunks, Kmax]   per-chunk label histograms / bases
   int64_t partial;       // float [BH, Kmax, slabs, 128] centroid partial sums
   int64_t w_hi;          // bf16  [BH, Jpad, 128]
   int64_t w_lo;          // bf16  [BH, Jpad, 128]
@@ -41,7 +39,6 @@ struct Workspace {
   int64_t total;
 };
 
-__host__ inline int sort_chunks(int64_t N) { return (int)ceil_div64(N, kSortChunk); }
 __host__ inline int pad_clusters(int64_t K) { return (int)align_up(K, 256); }   // W rows, whole 256-row blocks
 __host__ inline int max_runs(int64_t KC) { return (int)(KC / 2 + 2); }   // + one sentinel entry
 __host__ inline int max_qtiles(int64_t N, int64_t QC) { return (int)(ceil_div64(N, kAttnBM) + QC); }
@@ -60,7 +57,6 @@ __host__ inline Workspace workspace_layout(int64_t BH, int64_t N, int64_t QC, in
   const int64_t Kmax = QC > KC ? QC : KC;
   int64_t o = 0;
   auto take = [&](int64_t bytes) { int64_t at = o; o += align_up(bytes, 256); return at; };
-  w.chunk_hist = take(BH * sort_chunks(N) * Kmax * 4);
   w.partial = take(BH * Kmax * kCentroidSlabs * kHeadDim * 4);
   w.w_hi = take(BH * (int64_t)pad_clusters(Kmax) * kRowBytes);
   w.w_lo = take(BH * (int64_t)pad_clusters(Kmax) * kRowBytes);
