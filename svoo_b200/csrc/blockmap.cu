@@ -13,45 +13,75 @@
 
 namespace svoo {
 
-// Keys of one query cluster: (bf16 probability << 16) | (0xFFFF - cluster index), sorted descending
-// into kw[0 .. KCpad).
-template <int M>
-__device__ __forceinline__ void make_sorted_keys(const float* vw, uint32_t* kw, float tot, int KC, int KCpad, int lane) {
-  uint32_t v[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const int j = lane + 32 * m;
-    uint32_t kk = 0;
-    if (j < KC) {
-      const bf16 pb = __float2bfloat16_rn(__fdiv_rn(vw[j], tot));
-      kk = ((uint32_t)__bfloat16_as_ushort(pb) << 16) | (uint32_t)(0xFFFF - j);
-    }
-    v[m] = kk;
-  }
-  warp_sort_desc<M>(v, lane);
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const int t = lane + 32 * m;
-    if (t < KCpad) kw[t] = v[m];
-  }
+// One CTA = 8 consecutive query clusters of one head, one warp each; kM = key clusters per lane (KC <= 32 kM).
+//   * Scores, all 8 warps together: a thread multiplies one or two key centroids with the 8 query centroids; every
+//     (query, key) sum runs over d in ascending order, two query clusters to an instruction (f32x2).
+//   * The rest is per query cluster and runs in the 8 warps side by side: exp, the sequential sum (lane 0,
+//     the next shared-memory reads in flight), the probabilities as keys in registers.
+//   * Which clusters stay is a question of how many when the limits or the first probability decide
+//     (cap <= floor, or top_p below the largest probability): then the n-th largest key is found bit by bit
+//     (26 counts) and nothing is sorted.  Otherwise the keys are sorted and their prefix sums formed up to
+//     the first one above top_p.
+// 24 heads x 256 x 1024 clusters: 257 us with one query cluster to an instruction, a bitonic sort in every
+// case and unpipelined sums (of which scores 94, sort 42, sums 62).
+constexpr int kMapRows = 8;
+// Key clusters per pass of the score phase.
+__host__ __device__ constexpr int map_rows_pass(int M) { return 32 * M < 512 ? 32 * M : 512; }
+inline size_t map_smem_bytes(int M) {
+  const size_t keys = (size_t)kMapRows * 32 * M * 4, stages = 2 * (size_t)map_rows_pass(M) * 64;
+  return (size_t)kMapRows * kHeadDim * 4 + keys + (keys > stages ? keys : stages);              // at most 100 KB
 }
 
-// One CTA = 8 consecutive query clusters of one head, one warp each.  The score phase is shared:
-// a thread reads a key centroid once and accumulates its product with all 8 query centroids
-// (each (query, key) sum still runs over d in ascending order).  Everything after it -- exp,
-// the sequential sum, the sort, the sequential bf16 prefix sum -- is per query cluster and runs in
-// the 8 warps side by side, which is what the fixed summation orders leave to parallelise.
-constexpr int kMapRows = 8;
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t both(float v) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ void unpair(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 
+// x[0] + x[1] + ... + x[n - 1] in that order; x is 16-byte aligned and readable up to a multiple of 16 past n.
+__device__ __forceinline__ float ordered_sum(const float* x, int n) {
+  const float4* p = reinterpret_cast<const float4*>(x);
+  float tot = 0.f;
+  float4 a[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) a[i] = p[i];
+  int j = 0;
+  for (; j + 16 <= n; j += 16) {
+    float4 nxt[4];
+    const int q = j + 16 < n ? (j + 16) / 4 : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) nxt[i] = p[q + i];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      tot = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tot, a[i].x), a[i].y), a[i].z), a[i].w);
+      a[i] = nxt[i];
+    }
+  }
+  for (; j < n; ++j) tot = __fadd_rn(tot, x[j]);
+  return tot;
+}
+
+template <int kM>
 __global__ void __launch_bounds__(256, 2) block_map_kernel(const bf16* __restrict__ qc, const bf16* __restrict__ kc,
                                                         const int32_t* __restrict__ ksizes, uint8_t* __restrict__ map,
-                                                        int QC, int KC, int KCpad, float sqrt_d, float top_p,
+                                                        int QC, int KC, float sqrt_d, float top_p,
                                                         const __grid_constant__ HeadLimits lim) {
+  constexpr int kPad = 32 * kM, kRowsPass = map_rows_pass(kM), kJ = kRowsPass > 256 ? 2 : 1;
   extern __shared__ __align__(16) unsigned char map_sm[];
-  float* q_s = reinterpret_cast<float*>(map_sm);                       // [8][128]
-  float* val = q_s + kMapRows * kHeadDim;                              // [8][KCpad]: scores, weighted exps, prefix sums
-  uint32_t* key = reinterpret_cast<uint32_t*>(val + kMapRows * KCpad); // [8][KCpad]
-  __shared__ float red[8][kMapRows];
+  float* q_s = reinterpret_cast<float*>(map_sm);                       // [128][8]
+  float* val = q_s + kMapRows * kHeadDim;                              // [8][kPad]: scores, then weighted exps
+  uint32_t* key = reinterpret_cast<uint32_t*>(val + kMapRows * kPad);  // two stages of key centroids, then [8][kPad] sorted keys
   const int i0 = blockIdx.x * kMapRows, bh = blockIdx.y, tid = threadIdx.x;
   const int lane = tid % 32, warp = tid / 32;
   if (top_p >= 1.0f) {
@@ -61,117 +91,183 @@ __global__ void __launch_bounds__(256, 2) block_map_kernel(const bf16* __restric
   }
   for (int t = tid; t < kMapRows * kHeadDim; t += 256) {
     const int r = t / kHeadDim, d = t % kHeadDim;
-    q_s[t] = i0 + r < QC ? __bfloat162float(qc[((int64_t)bh * QC + i0 + r) * kHeadDim + d]) : 0.f;
+    q_s[d * kMapRows + r] = i0 + r < QC ? __bfloat162float(qc[((int64_t)bh * QC + i0 + r) * kHeadDim + d]) : 0.f;
   }
   __syncthreads();
 
-  float lmax[kMapRows];
+  // The key centroids pass through shared memory 32 dims of 512 rows at a time (64-byte rows, chunks
+  // XOR-swizzled by the row pair so that 8 lanes read 8 different bank groups), double buffered: read row by row
+  // from global memory, a warp's 16-byte loads touch 32 rows each and their latency was the score phase's time.
+  const uint32_t kbuf = smem_u32(key);
+  const int passes = (KC + kRowsPass - 1) / kRowsPass, stages = passes * 4;
+  auto load = [&](int s) {
+    const int base = s / 4 * kRowsPass, dim0 = s % 4 * 32;
+    const uint32_t dst = kbuf + (s & 1) * kRowsPass * 64;
+    for (int t = tid; t < kRowsPass * 4; t += 256) {
+      const int r = t >> 2, ch = t & 3;
+      cp_async16(dst + r * 64 + ((ch ^ ((r >> 1) & 3)) << 4),
+                 kc + ((int64_t)bh * KC + min(base + r, KC - 1)) * kHeadDim + dim0 + ch * 8, base + r < KC);
+    }
+    cp_async_commit();
+  };
+  load(0);
+  uint64_t acc[kJ][4];                                                 // [row of this thread][pair of query clusters]
+  for (int s = 0; s < stages; ++s) {
+    if (s + 1 < stages) {
+      load(s + 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    if (s % 4 == 0) {
 #pragma unroll
-  for (int r = 0; r < kMapRows; ++r) lmax[r] = -INFINITY;
-  for (int j = tid; j < KC; j += 256) {
-    const uint4* row = reinterpret_cast<const uint4*>(kc + ((int64_t)bh * KC + j) * kHeadDim);
-    float acc[kMapRows];
+      for (int x = 0; x < kJ; ++x)
 #pragma unroll
-    for (int r = 0; r < kMapRows; ++r) acc[r] = 0.f;
-#pragma unroll 2
-    for (int c = 0; c < 16; ++c) {
-      const uint4 v = __ldg(row + c);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-      float kv[8];
+        for (int p = 0; p < 4; ++p) acc[x][p] = 0;                     // two fp32 zeros
+    }
+    const unsigned char* kb = reinterpret_cast<const unsigned char*>(key) + (s & 1) * kRowsPass * 64;
+    if (tid < kRowsPass) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        kv[2 * e] = __low2float(h[e]);
-        kv[2 * e + 1] = __high2float(h[e]);
+      for (int ch = 0; ch < 4; ++ch) {
+        uint4 kv[kJ];
+#pragma unroll
+        for (int x = 0; x < kJ; ++x) {
+          const int r = tid + 256 * x;
+          kv[x] = *reinterpret_cast<const uint4*>(kb + r * 64 + ((ch ^ ((r >> 1) & 3)) << 4));
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const ulonglong2* qd = reinterpret_cast<const ulonglong2*>(q_s + (s % 4 * 32 + ch * 8 + e) * kMapRows);
+          const ulonglong2 qa = qd[0], qb = qd[1];
+          const uint64_t q2[4] = {qa.x, qa.y, qb.x, qb.y};
+#pragma unroll
+          for (int x = 0; x < kJ; ++x) {
+            // bf16 -> fp32: the low half of the word shifted up, or the high half masked
+            const uint32_t w = reinterpret_cast<const uint32_t*>(&kv[x])[e / 2];
+            const uint64_t k2 = both(__uint_as_float((e & 1) ? (w & 0xFFFF0000u) : (w << 16)));
+#pragma unroll
+            for (int p = 0; p < 4; ++p) acc[x][p] = add2(acc[x][p], mul2(q2[p], k2));
+          }
+        }
       }
+      if (s % 4 == 3) {
 #pragma unroll
-      for (int r = 0; r < kMapRows; ++r) {
+        for (int x = 0; x < kJ; ++x) {
+          const int j = s / 4 * kRowsPass + tid + 256 * x;
+          if (j < KC) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[r] = __fadd_rn(acc[r], __fmul_rn(q_s[r * kHeadDim + c * 8 + e], kv[e]));
+            for (int p = 0; p < 4; ++p) {
+              float lo, hi;
+              unpair(acc[x][p], lo, hi);
+              val[(2 * p) * kPad + j] = bf16_round(__fdiv_rn(bf16_round(lo), sqrt_d));
+              val[(2 * p + 1) * kPad + j] = bf16_round(__fdiv_rn(bf16_round(hi), sqrt_d));
+            }
+          }
+        }
       }
     }
-#pragma unroll
-    for (int r = 0; r < kMapRows; ++r) {
-      float sc = bf16_round(acc[r]);
-      sc = bf16_round(__fdiv_rn(sc, sqrt_d));
-      val[r * KCpad + j] = sc;
-      lmax[r] = fmaxf(lmax[r], sc);
-    }
+    __syncthreads();                                                   // the next load overwrites this stage's buffer
   }
-#pragma unroll
-  for (int r = 0; r < kMapRows; ++r) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lmax[r] = fmaxf(lmax[r], __shfl_xor_sync(0xffffffffu, lmax[r], o));
-    if (lane == 0) red[warp][r] = lmax[r];
-  }
-  __syncthreads();
 
   // ---- from here on: warp w works on query cluster i0 + w
   const int i = i0 + warp;
   if (i >= QC) return;
-  float* vw = val + warp * KCpad;
-  uint32_t* kw = key + warp * KCpad;
-  float mx = red[0][warp];
+  float* vw = val + warp * kPad;
+  uint32_t* kw = key + warp * kPad;
+  float mx = -INFINITY;
 #pragma unroll
-  for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red[w][warp]);
-  for (int j = lane; j < KC; j += 32) {
-    const float e = exp_f32_fixed(__fsub_rn(vw[j], mx));
-    vw[j] = __fmul_rn((float)ksizes[(int64_t)bh * KC + j], e);
+  for (int m = 0; m < kM; ++m)
+    if (lane + 32 * m < KC) mx = fmaxf(mx, vw[lane + 32 * m]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+  for (int m = 0; m < kM; ++m) {
+    const int j = lane + 32 * m;
+    float e = 0.f;
+    if (j < KC) e = __fmul_rn((float)ksizes[(int64_t)bh * KC + j], exp_f32_fixed(__fsub_rn(vw[j], mx)));
+    vw[j] = e;
   }
   __syncwarp();
   float tot = 0.f;
-  if (lane == 0) {                                   // j ascending; four values per shared-memory read
-    int j = 0;
-    if (KCpad >= 4)
-      for (; j + 4 <= KC; j += 4) {
-        const float4 t4 = *reinterpret_cast<const float4*>(vw + j);
-        tot = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tot, t4.x), t4.y), t4.z), t4.w);
-      }
-    for (; j < KC; ++j) tot = __fadd_rn(tot, vw[j]);
-    tot = fmaxf(tot, 1e-12f);
-  }
+  if (lane == 0) tot = fmaxf(ordered_sum(vw, KC), 1e-12f);             // j ascending
   tot = __shfl_sync(0xffffffffu, tot, 0);
-  switch (KCpad <= 32 ? 1 : KCpad / 32) {           // registers per lane
-    case 1: make_sorted_keys<1>(vw, kw, tot, KC, KCpad, lane); break;
-    case 2: make_sorted_keys<2>(vw, kw, tot, KC, KCpad, lane); break;
-    case 4: make_sorted_keys<4>(vw, kw, tot, KC, KCpad, lane); break;
-    case 8: make_sorted_keys<8>(vw, kw, tot, KC, KCpad, lane); break;
-    case 16: make_sorted_keys<16>(vw, kw, tot, KC, KCpad, lane); break;
-    default: make_sorted_keys<32>(vw, kw, tot, KC, KCpad, lane); break;
-  }
-  __syncwarp();
-  if (lane == 0) {                                   // r ascending; padding keys are zero probabilities
-    float run = 0.f;
-    int r = 0;
-    if (KCpad >= 4)
-      for (; r + 4 <= KCpad; r += 4) {
-        const uint4 k4 = *reinterpret_cast<const uint4*>(kw + r);
-        float4 o;
-        run = __fadd_rn(run, __uint_as_float(k4.x & 0xFFFF0000u)); o.x = bf16_round(run);
-        run = __fadd_rn(run, __uint_as_float(k4.y & 0xFFFF0000u)); o.y = bf16_round(run);
-        run = __fadd_rn(run, __uint_as_float(k4.z & 0xFFFF0000u)); o.z = bf16_round(run);
-        run = __fadd_rn(run, __uint_as_float(k4.w & 0xFFFF0000u)); o.w = bf16_round(run);
-        *reinterpret_cast<float4*>(vw + r) = o;
-      }
-    for (; r < KC; ++r) {
-      run = __fadd_rn(run, __uint_as_float(kw[r] & 0xFFFF0000u));
-      vw[r] = bf16_round(run);
+  // key of cluster j: (bf16 probability << 16) | (0xFFFF - j); descending keys = descending probability, ties by
+  // lower index
+  uint32_t v[kM], top = 0;
+#pragma unroll
+  for (int m = 0; m < kM; ++m) {
+    const int j = lane + 32 * m;
+    v[m] = 0;
+    if (j < KC) {
+      const bf16 pb = __float2bfloat16_rn(__fdiv_rn(vw[j], tot));
+      v[m] = ((uint32_t)__bfloat16_as_ushort(pb) << 16) | (uint32_t)(0xFFFF - j);
     }
+    top = max(top, v[m]);
   }
-  __syncwarp();
+  top = __reduce_max_sync(0xffffffffu, top);
+  // Position r of the descending order stays iff r < cap and (r < floor or r <= cut), cut = the first position
+  // whose bf16 prefix sum is above top_p (prefix sums do not decrease).
   const float p_b = bf16_round(top_p);
-  const int preserve = lim.preserve[bh], cap = lim.cap[bh];
+  const int preserve = max(lim.preserve[bh], 0), cap = max(min(lim.cap[bh], KC), 0);
   uint8_t* out = map + ((int64_t)bh * QC + i) * KC;
-  for (int r = lane; r < KC; r += 32) {
-    bool remove = (r >= 1) && (vw[r - 1] > p_b);
-    if (r < preserve) remove = false;
-    if (r >= cap) remove = true;
-    out[0xFFFF - (kw[r] & 0xFFFFu)] = remove ? 0 : 1;
+  int n = cap;                                          // kept positions
+  uint32_t thr = 0;
+  if (cap > preserve && __uint_as_float(top & 0xFFFF0000u) > p_b) n = min(cap, max(preserve, 1));    // cut = 0
+  if (cap <= preserve || __uint_as_float(top & 0xFFFF0000u) > p_b) {
+    if (n > 0 && n < KC) {                              // thr = the n-th largest key (keys are distinct)
+#pragma unroll 1
+      for (int bit = 31; bit >= 0; --bit) {
+        if (bit == 15) {                                // 0xFFFF - j with j < 1024: bits 10 to 15 are set in every key
+          thr |= 0xFC00u;
+          bit = 9;
+        }
+        const uint32_t cand = thr | (1u << bit);
+        int cnt = 0;
+#pragma unroll
+        for (int m = 0; m < kM; ++m) cnt += v[m] >= cand;
+        if ((int)__reduce_add_sync(0xffffffffu, (unsigned)cnt) >= n) thr = cand;
+      }
+    }
+  } else {
+    uint32_t sorted[kM];
+#pragma unroll
+    for (int m = 0; m < kM; ++m) sorted[m] = v[m];
+    warp_sort_desc<kM>(sorted, lane);
+#pragma unroll
+    for (int m = 0; m < kM; ++m) kw[lane + 32 * m] = sorted[m];
+    __syncwarp();
+    int cut = cap;                                      // past the cap nothing stays
+    if (lane == 0) {                                    // r ascending, eight per step
+      float run = 0.f;
+      for (int r = 0; r < cap && cut == cap; r += 8) {
+        const uint4 a = *reinterpret_cast<const uint4*>(kw + r), b = *reinterpret_cast<const uint4*>(kw + r + 4);
+        const uint32_t k8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        float pre[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          run = __fadd_rn(run, __uint_as_float(k8[u] & 0xFFFF0000u));
+          pre[u] = run;
+        }
+#pragma unroll
+        for (int u = 7; u >= 0; --u)
+          if (bf16_round(pre[u]) > p_b) cut = min(r + u, cap);
+      }
+    }
+    cut = __shfl_sync(0xffffffffu, cut, 0);
+    n = min(cap, max(preserve, cut + 1));
+    if (n > 0 && n < KC) thr = kw[n - 1];
+  }
+#pragma unroll
+  for (int m = 0; m < kM; ++m) {
+    const int j = lane + 32 * m;
+    if (j < KC) out[j] = n > 0 && v[m] >= thr ? 1 : 0;
   }
 }
 
 // ---------------------------------------------------------------------------------------------
 // The two index lists of the attention kernels, in one launch: blocks [0, BH) write the query tiles of
-// one head each, the blocks after them the key-row runs of eight (head, query cluster) rows each.
+// one head each, the blocks after them the key-row runs of eight query clusters of a head each.
 // ---------------------------------------------------------------------------------------------
 // Query tiles of every non-empty query cluster, in cluster order; thread i owns clusters
 // [kPer i, kPer (i + 1)).  Tiles of kRows rows; with kSplit (kRows = 256) a remainder of up to 128 rows goes
@@ -233,59 +329,106 @@ __device__ void build_qtiles(const int32_t* __restrict__ off, int4* __restrict__
 // kEar: the K/V tensors are the cluster-ordered rows of all heads followed by the centroid rows of all
 // heads ([BH*S + BH*KC, 128]), and the list ends with ONE more run, the KC centroid rows of the head
 // (the attention kernels mask the centroids of the selected clusters).
+// The block's rows belong to one head, whose offsets (and a bit per non-empty cluster) are staged in shared
+// memory.  Lane l of a row's warp reads its own 32 map bytes, keeps them as a 32-bit mask and walks the runs
+// of that mask twice: their rows are summed, a scan over the lanes gives the first run and virtual row, and
+// they are written.  The instruction count is what this costs: about 450 per row; with a vote for every 32
+// clusters and 64-bit masks 2,300 (24 heads x 258 rows x 1,026 clusters: 36 us), with a scan for every 32
+// clusters 43 us.
+constexpr int kListRows = kListThreads / 32;
 template <bool kEar>
 __device__ void build_runs(const uint8_t* __restrict__ map, const int32_t* __restrict__ k_offsets, int2* __restrict__ runs,
-                           int32_t* __restrict__ nruns, int32_t* __restrict__ head_work, int row, int BH, int S, int QC, int KC,
-                           int max_runs) {
-  const int lane = threadIdx.x % 32;
-  const int bh = row / QC;
-  const uint8_t* m = map + (int64_t)row * KC;
+                           int32_t* __restrict__ nruns, int32_t* __restrict__ head_work, int bh, int i0, int BH, int S, int QC,
+                           int KC, int max_runs) {
+  constexpr int kMask = 1024;                                          // clusters in the lanes' masks; the rest: lane 31
+  __shared__ int32_t off_s[SVOO_MAX_ATTN_CLUSTERS + 1];
+  __shared__ uint32_t filled[kMask / 32];
   const int32_t* off = k_offsets + (int64_t)bh * (KC + 1);
-  int2* out = runs + (int64_t)row * max_runs;
-  const int limit = max_runs - (kEar ? 2 : 1);
-  bool carry = false;                                    // the cluster before this chunk is in a run
-  int n = 0, vbeg = 0;                                   // runs and selected rows so far
-  constexpr int kU = 4;
-  for (int base = 0; base < KC; base += 32 * kU) {       // the loads of kU chunks are in flight together
-    int first[kU], size[kU];
+  for (int j = threadIdx.x; j <= KC; j += kListThreads) off_s[j] = off[j];
+  const int r = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int64_t row = (int64_t)bh * QC + min(i0 + r, QC - 1);
+  const uint8_t* m = map + row * KC;
+  // bytes [32 lane, 32 lane + 32) of the row as nine aligned words, of which only those that hold one of them are read
+  const int j0 = lane * 32, bytes = max(min(KC - j0, 32), 0);
+  const uintptr_t at = reinterpret_cast<uintptr_t>(m + j0);
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
+  const int skew = (int)(at & 3);
+  uint32_t w[9];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int j = base + u * 32 + lane;
-      first[u] = size[u] = 0;
-      if (j < KC) {
-        first[u] = off[j];
-        size[u] = m[j] != 0 ? off[j + 1] - first[u] : 0;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      int incl = size[u];
-#pragma unroll
-      for (int s = 1; s < 32; s <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, incl, s);
-        if (lane >= s) incl += o;
-      }
-      const bool act = size[u] > 0;
-      const unsigned bal = __ballot_sync(0xffffffffu, act);
-      const unsigned starts = bal & ~((bal << 1) | (carry ? 1u : 0u));
-      if ((starts >> lane) & 1u) {
-        const int r = n + __popc(starts & ((1u << lane) - 1u));
-        if (r < limit) out[r] = make_int2(first[u], vbeg + incl - size[u]);
-      }
-      n += __popc(starts);
-      vbeg += __shfl_sync(0xffffffffu, incl, 31);
-      carry = (bal >> 31) != 0;
-    }
+  for (int i = 0; i < 9; ++i) w[i] = 4 * i < bytes + skew && bytes > 0 ? __ldg(words + i) : 0;
+  __syncthreads();
+  for (int t = r; t < kMask / 32; t += kListRows) {
+    const int j = t * 32 + lane;
+    const unsigned word = __ballot_sync(0xffffffffu, j < KC && off_s[min(j + 1, KC)] > off_s[min(j, KC)]);
+    if (lane == 0) filled[t] = word;
   }
-  if (lane == 0) {
-    n = min(n, limit);
-    if (kEar) {
-      out[n++] = make_int2((BH - bh) * S + bh * KC, vbeg);           // the head's centroid rows
-      vbeg += KC;
+  __syncthreads();
+  if (i0 + r >= QC) return;
+  uint32_t sel = 0;                                                    // bit b: cluster j0 + b, selected and not empty
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t x = __funnelshift_r(w[i], w[i + 1], 8 * skew);
+    uint32_t nz = ((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | x) & 0x80808080u;       // top bit of every byte that is not zero
+    nz = (nz >> 7) * 0x10204080u >> 28;                                      // the four of them side by side
+    sel |= nz << (4 * i);
+  }
+  sel &= filled[lane];
+  int2* out = runs + row * max_runs;
+  const int limit = max_runs - (kEar ? 2 : 1);
+  // [b, e) = the first run of `rest`; what is left of it
+  auto next_run = [](uint32_t& rest, int& b, int& e) {
+    b = __ffs(rest) - 1;
+    const uint32_t gap = ~(rest >> b);
+    e = gap ? b + __ffs(gap) - 1 : 32;
+    rest = e >= 32 ? 0u : rest >> e << e;
+  };
+  int n = 0, sum = 0;
+  for (uint32_t rest = sel; rest;) {
+    int b, e;
+    next_run(rest, b, e);
+    sum += off_s[j0 + e] - off_s[j0 + b];
+    ++n;
+  }
+  // the lane's first run may continue the one of the lane before
+  const uint32_t before = __shfl_up_sync(0xffffffffu, sel >> 31, 1);
+  const bool joined = lane > 0 && before && (sel & 1);
+  n -= joined;
+  int n_incl = n, s_incl = sum;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, n_incl, s), b = __shfl_up_sync(0xffffffffu, s_incl, s);
+    if (lane >= s) { n_incl += a; s_incl += b; }
+  }
+  int pos = n_incl - n - joined, vbeg = s_incl - sum;
+  bool skip = joined;
+  for (uint32_t rest = sel; rest;) {
+    int b, e;
+    next_run(rest, b, e);
+    if (!skip && pos < limit) out[pos] = make_int2(off_s[j0 + b], vbeg);
+    skip = false;
+    ++pos;
+    vbeg += off_s[j0 + e] - off_s[j0 + b];
+  }
+  if (lane == 31) {
+    int k = n_incl, rows_sel = s_incl;
+    bool in_run = sel >> 31;
+    for (int j = kMask; j < KC; ++j) {                                 // the text blocks of a 1024-cluster layer
+      const int size = m[j] != 0 ? off_s[j + 1] - off_s[j] : 0;
+      if (size > 0 && !in_run) {
+        if (k < limit) out[k] = make_int2(off_s[j], rows_sel);
+        ++k;
+      }
+      in_run = size > 0;
+      rows_sel += size;
     }
-    out[n] = make_int2(0, vbeg);
-    nruns[row] = n;
-    atomicAdd(&head_work[bh], (vbeg + 127) / 128);
+    k = min(k, limit);
+    if (kEar) {
+      out[k++] = make_int2((BH - bh) * S + bh * KC, rows_sel);         // the head's centroid rows
+      rows_sel += KC;
+    }
+    out[k] = make_int2(0, rows_sel);
+    nruns[row] = k;
+    atomicAdd(&head_work[bh], (rows_sel + 127) / 128);
   }
 }
 
@@ -294,13 +437,17 @@ __global__ void __launch_bounds__(kListThreads) attn_lists_kernel(
     const int32_t* __restrict__ q_offsets, int4* __restrict__ qtiles, int32_t* __restrict__ nqtiles, int max_tiles,
     const uint8_t* __restrict__ map, const int32_t* __restrict__ k_offsets, int2* __restrict__ runs,
     int32_t* __restrict__ nruns, int32_t* __restrict__ sched, int32_t* __restrict__ head_order, int BH, int S, int QC, int KC,
-    int max_runs) {
+    int max_runs, bool ordered) {
   if ((int)blockIdx.x < BH) {
     const int bh = blockIdx.x;
     build_qtiles<kRows, kSplit>(q_offsets + (int64_t)bh * (QC + 1), qtiles + (int64_t)bh * max_tiles, nqtiles + 2 * bh, QC, max_tiles);
   } else {
-    const int row = (blockIdx.x - BH) * (kListThreads / 32) + threadIdx.x / 32;
-    if (row < BH * QC) build_runs<kEar>(map, k_offsets, runs, nruns, sched + 1, row, BH, S, QC, KC, max_runs);
+    const int per_head = (QC + kListRows - 1) / kListRows, b = blockIdx.x - BH;
+    build_runs<kEar>(map, k_offsets, runs, nruns, sched + 1, b / per_head, b % per_head * kListRows, BH, S, QC, KC, max_runs);
+  }
+  if (!ordered) {
+    if ((int)blockIdx.x < BH && threadIdx.x == 0) head_order[blockIdx.x] = blockIdx.x;
+    return;
   }
   // The last block to finish orders the heads by their selected key tiles (summed over query clusters).
   __shared__ bool last;
@@ -312,15 +459,16 @@ __global__ void __launch_bounds__(kListThreads) attn_lists_kernel(
   __syncthreads();
   if (!last) return;
   __threadfence();
+  constexpr int kMaxOrdered = 1024;                      // with more heads any order ends evenly
+  __shared__ int work[kMaxOrdered];
+  for (int h = threadIdx.x; h < min(BH, kMaxOrdered); h += kListThreads) work[h] = __ldcg(sched + 1 + h);
+  __syncthreads();
   for (int h = threadIdx.x; h < BH; h += kListThreads) {
     int rank = h;
-    if (BH <= 1024) {                                    // more heads: any order ends evenly
-      const int mine = __ldcg(sched + 1 + h);
+    if (BH <= kMaxOrdered) {
+      const int mine = work[h];
       rank = 0;
-      for (int g = 0; g < BH; ++g) {
-        const int w = __ldcg(sched + 1 + g);
-        rank += w > mine || (w == mine && g < h);
-      }
+      for (int g = 0; g < BH; ++g) rank += work[g] > mine || (work[g] == mine && g < h);
     }
     head_order[rank] = h;
   }
@@ -334,14 +482,21 @@ cudaError_t launch_block_map(const void* qc, const void* kc, const int32_t* ksiz
     lim.preserve[h] = h < BH ? preserve_host[h] : 0;
     lim.cap[h] = h < BH ? cap_host[h] : (int32_t)KC;
   }
-  int KCpad = 2;
-  while (KCpad < KC) KCpad <<= 1;
-  const size_t smem = (size_t)kMapRows * (kHeadDim + 2 * KCpad) * 4;           // at most 68 KB (1024 clusters)
-  cudaError_t e = cudaFuncSetAttribute(block_map_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);
+  // key clusters per lane: the next power of two
+  int M = 1;
+  while (32 * M < KC) M <<= 1;
+  auto* kernel = M == 1   ? &block_map_kernel<1>
+                 : M == 2 ? &block_map_kernel<2>
+                 : M == 4 ? &block_map_kernel<4>
+                 : M == 8 ? &block_map_kernel<8>
+                 : M == 16 ? &block_map_kernel<16>
+                           : &block_map_kernel<32>;
+  const size_t smem = map_smem_bytes(M);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)map_smem_bytes(32));
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)ceil_div64(QC, kMapRows), (unsigned)BH);
-  block_map_kernel<<<grid, 256, smem, st>>>((const bf16*)qc, (const bf16*)kc, ksizes, map, (int)QC, (int)KC, KCpad,
-                                            (float)sqrt((double)kHeadDim), top_p, lim);
+  kernel<<<grid, 256, smem, st>>>((const bf16*)qc, (const bf16*)kc, ksizes, map, (int)QC, (int)KC,
+                                  (float)sqrt((double)kHeadDim), top_p, lim);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -395,6 +550,7 @@ cudaError_t launch_append_text_blocks(const uint8_t* map, const int32_t* q_off, 
   return cudaGetLastError();
 }
 
+// A grid of up to 256 query clusters starts in one wave, whatever the order of the heads.
 // tile_rows: 128 (mma.sync kernel) or 256; split: single tiles in their own list.  ear: with the head's
 // centroid run (256-row tiles only).
 cudaError_t launch_attn_lists(const int32_t* q_offsets, int4* qtiles, int32_t* nqtiles, const uint8_t* map,
@@ -403,9 +559,9 @@ cudaError_t launch_attn_lists(const int32_t* q_offsets, int4* qtiles, int32_t* n
   auto* kernel = tile_rows == 128 ? &attn_lists_kernel<128, false, false>
                  : ear ? (split ? &attn_lists_kernel<256, true, true> : &attn_lists_kernel<256, false, true>)
                        : (split ? &attn_lists_kernel<256, true, false> : &attn_lists_kernel<256, false, false>);
-  const int64_t blocks = BH + ceil_div64(BH * QC, kListThreads / 32);
+  const int64_t blocks = BH + BH * ceil_div64(QC, kListRows);
   kernel<<<(unsigned)blocks, kListThreads, 0, st>>>(q_offsets, qtiles, nqtiles, max_qtiles(S, QC), map, k_offsets, runs, nruns,
-                                                   sched, head_order, (int)BH, (int)S, (int)QC, (int)KC, max_runs);
+                                                   sched, head_order, (int)BH, (int)S, (int)QC, (int)KC, max_runs, BH * QC > 256);
   count_launches(1);
   return cudaGetLastError();
 }
