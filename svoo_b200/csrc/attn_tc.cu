@@ -559,9 +559,10 @@ cudaError_t launch_sparse_attn_tc(const void* q, const void* k, const void* v, v
   // tiles per head: of at least 129 rows each, or a cluster's whole 256-row tiles and its remainder
   const int per_head = (int)(split ? S / (tc::kBM + 1) : S / (2 * tc::kBM) + QC);
   if (per_head > 0) {
-    const bool gather = short_key_runs(S, KC);
-    auto* kernel = ear ? (gather ? &tc::sparse_attn_tc_kernel<true, true> : &tc::sparse_attn_tc_kernel<true, false>)
-                       : (gather ? &tc::sparse_attn_tc_kernel<false, true> : &tc::sparse_attn_tc_kernel<false, false>);
+    // EAR layers end every key list with a run of all centroids and stay with TMA
+    auto* kernel = ear ? &tc::sparse_attn_tc_kernel<true, false>
+                   : short_key_runs(S, KC) ? &tc::sparse_attn_tc_kernel<false, true>
+                                           : &tc::sparse_attn_tc_kernel<false, false>;
     const int smem = ear ? tc::AttnSmem<true>::kBytes : tc::AttnSmem<false>::kBytes;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
