@@ -33,143 +33,178 @@ __global__ void gather_rows_kernel(const bf16* __restrict__ x, const int32_t* __
 }
 
 // ---------------------------------------------------------------------------------------
-// Prologue: P = bf16(own . form^T), Phat = P / sqrt(sum P^2 + 1e-8), W = Phat . form -> (hi, lo) bf16.
-// The norm of a row is one number, so W = (P . form) / norm, and P, being bf16, is an exact operand of the
-// second product: one walk over `form` does both, the scores of 16 form rows going from accumulators to
-// A fragments in registers.  (svoo/co_clustering.py:2427-2428 and svoo/kernels/triton/l2norm.py:36-41)
-//
-// One CTA = 16 rows j of one head; its 8 warps split the form rows, 16 at a time, each with a cp.async ring of
-// its own (no CTA-wide barrier in the loop), and their partial W are added in warp order.  The problem is a
-// few MFLOP per head: its time is a chain of latencies.  With two walks over 64-row chunks behind CTA barriers
-// and Phat as three bf16 terms, mean of both sides: 24 heads x 256 / 1024 clusters 60 us, 12 x 100 / 500 13 us.
+// Prologue: P = bf16(own . form^T), Phat = P / sqrt(sum P^2 + 1e-8) (fp32),
+//           W = Phat . form (fp32) -> (hi, lo) bf16.     One CTA = 16 rows j of one head.
+// Both products run on mma.sync (m16n8k16, fp32 accumulation): the problem is a few MFLOP
+// per head and latency-bound, so the point is the short dependency chain, not throughput.
+// `form` is streamed twice through a double-buffered shared-memory ring of 64-row chunks
+// (cp.async).  Phat (fp32) enters the second product as three bf16 terms hi + mid + lo,
+// which carries 24 mantissa bits, so W matches an fp32 product to rounding.
+// (svoo/co_clustering.py:2427-2428 and svoo/kernels/triton/l2norm.py:36-41)
 // ---------------------------------------------------------------------------------------
 constexpr int kProR = 16;            // own rows per CTA
-constexpr int kProWarps = 8, kProStages = 3;
-constexpr int kProTile = 16 * kRowBytes;                 // 16 form rows
-constexpr int kProRedStride = kHeadDim + 4;              // floats
-constexpr int kProSmem = kProR * kRowBytes + kProWarps * kProStages * kProTile;
-static_assert(kProWarps * kProR * kProRedStride * 4 <= kProWarps * kProStages * kProTile, "the partial sums reuse the rings");
+constexpr int kProC = 64;            // form rows per chunk
 
-__global__ void __launch_bounds__(32 * kProWarps, 2) profile_prologue_kernel(
+__host__ __device__ inline int pro_kround(int K) { return (K + kProC - 1) / kProC * kProC; }
+__host__ __device__ inline int pro_p_stride(int K) { return pro_kround(K) + 4; }       // floats
+__host__ __device__ inline int pro_hat_stride(int K) { return pro_kround(K) + 8; }     // bf16: 16 bytes past a multiple of 128
+inline size_t pro_smem_bytes(int K) {
+  return (size_t)kProR * kRowBytes + 2 * (size_t)kProC * kRowBytes + (size_t)kProR * pro_p_stride(K) * 4 +
+         3 * (size_t)kProR * pro_hat_stride(K) * 2;
+}
+
+__global__ void __launch_bounds__(256) profile_prologue_kernel(
     const bf16* __restrict__ own, const bf16* __restrict__ form, bf16* __restrict__ w_hi,
     bf16* __restrict__ w_lo, int J, int K, int Jpad) {
   extern __shared__ __align__(128) unsigned char pro_sm[];
-  __shared__ float ss_s[kProWarps][kProR];
   pdl_trigger();
+  pdl_wait();                                           // the centroids come from the previous kernel
   const int bh = blockIdx.y, j0 = blockIdx.x * kProR;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row = tid >> 4, ch = tid & 15;               // of the 16 x 128 result: 8 dims per thread
-  const int64_t o = ((int64_t)bh * Jpad + j0 + row) * kHeadDim + ch * 8;
-  pdl_wait();                                            // the centroids come from the previous kernel, and W was read before it
-  if (j0 >= J) {                                         // padding rows of W: zeros
-    *reinterpret_cast<uint4*>(w_hi + o) = make_uint4(0, 0, 0, 0);
-    *reinterpret_cast<uint4*>(w_lo + o) = make_uint4(0, 0, 0, 0);
+  if (j0 >= J) {                                        // padding rows of W: zeros
+    const int d = tid & 127, rg = tid >> 7;
+    for (int r = rg * 8; r < rg * 8 + 8; ++r)
+      if (j0 + r < Jpad) {
+        w_hi[((int64_t)bh * Jpad + j0 + r) * kHeadDim + d] = __float2bfloat16_rn(0.f);
+        w_lo[((int64_t)bh * Jpad + j0 + r) * kHeadDim + d] = __float2bfloat16_rn(0.f);
+      }
     return;
   }
-  const uint32_t own_s = smem_u32(pro_sm);
-  const uint32_t ring = own_s + kProR * kRowBytes + warp * kProStages * kProTile;
+  const int pstride = pro_p_stride(K), hstride = pro_hat_stride(K);
+  unsigned char* own_p = pro_sm;                                    // [16][128] bf16, swizzled
+  unsigned char* form_p = own_p + kProR * kRowBytes;                // 2 x [64][128] bf16, swizzled
+  float* p_s = reinterpret_cast<float*>(form_p + 2 * kProC * kRowBytes);       // [16][pstride]
+  bf16* hat = reinterpret_cast<bf16*>(p_s + kProR * pstride);                  // 3 x [16][hstride]
+  const uint32_t own_s = smem_u32(own_p), form_s = smem_u32(form_p), hat_s = smem_u32(hat);
   const bf16* form_b = form + (int64_t)bh * K * kHeadDim;
-  const int tiles = (K + 15) / 16;
-  auto load = [&](int t, int st) {                       // rows past K arrive as zeros
-    if (t < tiles) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = 2 * i + (lane >> 4), c = lane & 15, k = t * 16 + r;
-        cp_async16(ring + st * kProTile + swz(r, c), form_b + (int64_t)min(k, K - 1) * kHeadDim + c * 8, k < K);
-      }
-    }
-    cp_async_commit();
-  };
-  cp_async16(own_s + swz(row, ch), own + ((int64_t)bh * J + min(j0 + row, J - 1)) * kHeadDim + ch * 8, j0 + row < J);
-  cp_async_commit();
-#pragma unroll
-  for (int st = 0; st < kProStages - 1; ++st) load(warp + st * kProWarps, st);
-  cp_async_wait<kProStages - 1>();                       // own rows
-  __syncthreads();
-  uint32_t qa[8][4];
-#pragma unroll
-  for (int ks = 0; ks < 8; ++ks) ldmatrix_x4(qa[ks], own_s + swz((lane % 8) + ((lane / 8) % 2) * 8, ks * 2 + lane / 16));
+  const int nch = (K + kProC - 1) / kProC;
 
-  float wacc[16][4], ss[2] = {0.f, 0.f};
+  auto load_chunk = [&](int c, int buf) {               // rows past K arrive as zeros
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) wacc[i][e] = 0.f;
-  int st = 0;
-  for (int t = warp; t < tiles; t += kProWarps) {
-    cp_async_wait<kProStages - 2>();
-    __syncwarp();                                        // every lane's copies of this tile, and all reads of the stage refilled next
-    const uint32_t f = ring + st * kProTile;
-    load(t + (kProStages - 1) * kProWarps, st == 0 ? kProStages - 1 : st - 1);
-    float acc[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      uint32_t b[4];
-      ldmatrix_x4(b, f + swz((lane % 8) + (lane / 16) * 8, ks * 2 + ((lane / 8) % 2)));
-      mma_bf16(acc[0], qa[ks], b[0], b[1]);
-      mma_bf16(acc[1], qa[ks], b[2], b[3]);
+    for (int pass = 0; pass < 4; ++pass) {
+      const int i = tid + pass * 256, row = i >> 4, ch = i & 15;
+      const int k = c * kProC + row;
+      cp_async16(form_s + buf * (kProC * kRowBytes) + swz(row, ch),
+                 form_b + (int64_t)min(k, K - 1) * kHeadDim + ch * 8, k < K);
     }
-    // torch.matmul of bf16 tensors returns bf16
-    uint32_t a[4];
+  };
+  {
+    const int row = tid >> 4, ch = tid & 15;
+    const int j = j0 + row;
+    cp_async16(own_s + swz(row, ch), own + ((int64_t)bh * J + min(j, J - 1)) * kHeadDim + ch * 8, j < J);
+  }
+  load_chunk(0, 0);
+  cp_async_commit();
+
+  // ---- sweep 1: P[16][K]; warps 0..3 take 16 form rows of the chunk each
+  uint32_t qa[8][4];
+  for (int c = 0; c < nch; ++c) {
+    if (c + 1 < nch) load_chunk(c + 1, (c + 1) & 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    if (warp < 4) {
+      if (c == 0) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+        for (int ks = 0; ks < 8; ++ks)
+          ldmatrix_x4(qa[ks], own_s + swz((lane % 8) + ((lane / 8) % 2) * 8, ks * 2 + lane / 16));
+      }
+      const uint32_t f = form_s + (c & 1) * (kProC * kRowBytes);
+      float acc[2][4];
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const float x = bf16_round(acc[i][2 * half]), y = bf16_round(acc[i][2 * half + 1]);
-        ss[half] = fmaf(x, x, ss[half]);
-        ss[half] = fmaf(y, y, ss[half]);
-        a[2 * i + half] = pack_bf16x2(x, y);
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        uint32_t b[4];
+        ldmatrix_x4(b, f + swz(warp * 16 + (lane % 8) + (lane / 16) * 8, ks * 2 + ((lane / 8) % 2)));
+        mma_bf16(acc[0], qa[ks], b[0], b[1]);
+        mma_bf16(acc[1], qa[ks], b[2], b[3]);
       }
 #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-      uint32_t b[4];
-      ldmatrix_x4_trans(b, f + swz((lane % 8) + ((lane / 8) % 2) * 8, g * 2 + lane / 16));
-      mma_bf16(wacc[2 * g], a, b[0], b[1]);
-      mma_bf16(wacc[2 * g + 1], a, b[2], b[3]);
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {                   // torch.matmul of bf16 tensors returns bf16
+          const int row = lane / 4 + (e >> 1) * 8;
+          const int k = c * kProC + warp * 16 + nt * 8 + 2 * (lane % 4) + (e & 1);
+          p_s[row * pstride + k] = bf16_round(acc[nt][e]);
+        }
     }
-    st = st == kProStages - 1 ? 0 : st + 1;
+    __syncthreads();
   }
-  cp_async_wait<0>();
+  load_chunk(0, 0);                                     // first chunk of sweep 2, in flight during the norms
+  cp_async_commit();
+
+  // ---- row norms (16 threads per row, fixed order), Phat = P / norm split into three bf16 terms
+  {
+    const int row = tid >> 4, sub = tid & 15;
+    const int kr = pro_kround(K);
+    float ss = 0.f;
+    for (int k = sub; k < kr; k += 16) { const float x = p_s[row * pstride + k]; ss = fmaf(x, x, ss); }
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    ss[half] += __shfl_xor_sync(0xffffffffu, ss[half], 1);
-    ss[half] += __shfl_xor_sync(0xffffffffu, ss[half], 2);
-    if (lane % 4 == 0) ss_s[warp][lane / 4 + 8 * half] = ss[half];
+    for (int o = 8; o >= 1; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float nr = sqrtf(ss + 1e-8f);
+    for (int k = sub; k < kr; k += 16) {
+      const float x = p_s[row * pstride + k] / nr;
+      const bf16 h = __float2bfloat16_rn(x);
+      const float r1 = x - __bfloat162float(h);
+      const bf16 m = __float2bfloat16_rn(r1);
+      const bf16 l = __float2bfloat16_rn(r1 - __bfloat162float(m));
+      hat[(0 * kProR + row) * hstride + k] = h;
+      hat[(1 * kProR + row) * hstride + k] = m;
+      hat[(2 * kProR + row) * hstride + k] = l;
+    }
   }
-  __syncthreads();                                       // every warp is done with its ring
-  float* red = reinterpret_cast<float*>(pro_sm + kProR * kRowBytes);           // [warp][16][132]
+
+  // ---- sweep 2: W[16][128] = sum_k Phat[r][k] form[k][d]; warp w owns dims 16w .. 16w+15
+  float wacc[3][2][4];
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
+  for (int t = 0; t < 3; ++t)
 #pragma unroll
-    for (int half = 0; half < 2; ++half)
-      *reinterpret_cast<float2*>(red + (warp * kProR + lane / 4 + 8 * half) * kProRedStride + i * 8 + 2 * (lane % 4)) =
-          make_float2(wacc[i][2 * half], wacc[i][2 * half + 1]);
-  __syncthreads();
-  float sum = 0.f, v[8];
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-  for (int d = 0; d < 8; ++d) v[d] = 0.f;
+      for (int e = 0; e < 4; ++e) wacc[t][i][e] = 0.f;
+  for (int c = 0; c < nch; ++c) {
+    if (c + 1 < nch) load_chunk(c + 1, (c + 1) & 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    const uint32_t f = form_s + (c & 1) * (kProC * kRowBytes);
 #pragma unroll
-  for (int w = 0; w < kProWarps; ++w) {
-    sum += ss_s[w][row];
-    const float4* p = reinterpret_cast<const float4*>(red + (w * kProR + row) * kProRedStride + ch * 8);
-    const float4 x = p[0], y = p[1];
-    v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-    v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t b[4];
+      ldmatrix_x4_trans(b, f + swz(kk * 16 + (lane % 8) + ((lane / 8) % 2) * 8, warp * 2 + lane / 16));
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        uint32_t a[4];
+        const int arow = (lane % 8) + ((lane / 8) % 2) * 8;
+        const int acol = c * kProC + kk * 16 + (lane / 16) * 8;
+        ldmatrix_x4(a, hat_s + (uint32_t)(((t * kProR + arow) * hstride + acol) * 2));
+        mma_bf16(wacc[t][0], a, b[0], b[1]);
+        mma_bf16(wacc[t][1], a, b[2], b[3]);
+      }
+    }
+    __syncthreads();
   }
-  const float nr = sqrtf(sum + 1e-8f);
-  uint32_t hi[4], lo[4];
 #pragma unroll
-  for (int d = 0; d < 4; ++d) {
-    const float x = v[2 * d] / nr, y = v[2 * d + 1] / nr;
-    hi[d] = pack_bf16x2(x, y);
-    lo[d] = pack_bf16x2(x - bf16_round(x), y - bf16_round(y));
-  }
-  *reinterpret_cast<uint4*>(w_hi + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-  *reinterpret_cast<uint4*>(w_lo + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int j = j0 + lane / 4 + half * 8;
+      if (j < Jpad) {
+        float v0 = wacc[0][nt][half * 2] + (wacc[1][nt][half * 2] + wacc[2][nt][half * 2]);
+        float v1 = wacc[0][nt][half * 2 + 1] + (wacc[1][nt][half * 2 + 1] + wacc[2][nt][half * 2 + 1]);
+        if (j >= J) v0 = v1 = 0.f;
+        const bf16 h0 = __float2bfloat16_rn(v0), h1 = __float2bfloat16_rn(v1);
+        const bf16 l0 = __float2bfloat16_rn(v0 - __bfloat162float(h0)), l1 = __float2bfloat16_rn(v1 - __bfloat162float(h1));
+        const int64_t o = ((int64_t)bh * Jpad + j) * kHeadDim + warp * 16 + nt * 8 + 2 * (lane % 4);
+        __nv_bfloat162 hv, lv;
+        hv.x = h0; hv.y = h1; lv.x = l0; lv.y = l1;
+        *reinterpret_cast<__nv_bfloat162*>(w_hi + o) = hv;
+        *reinterpret_cast<__nv_bfloat162*>(w_lo + o) = lv;
+      }
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -495,12 +530,13 @@ cudaError_t launch_gather_rows(const void* x, const int32_t* idx, void* out, int
 cudaError_t launch_prologue(const void* own, const void* form, void* w_hi, void* w_lo, int64_t BH, int64_t J,
                             int64_t K, cudaStream_t st) {
   const int Jpad = pad_clusters(J);
-  cudaError_t e = cudaFuncSetAttribute(profile_prologue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProSmem);
+  const size_t smem = pro_smem_bytes((int)K);
+  cudaError_t e = cudaFuncSetAttribute(profile_prologue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)(Jpad / kProR), (unsigned)BH);
   count_launches(1);
-  return launch_pdl(profile_prologue_kernel, grid, dim3(32 * kProWarps), (size_t)kProSmem, st, (const bf16*)own,
-                    (const bf16*)form, (bf16*)w_hi, (bf16*)w_lo, (int)J, (int)K, Jpad);
+  return launch_pdl(profile_prologue_kernel, grid, dim3(256), smem, st, (const bf16*)own, (const bf16*)form, (bf16*)w_hi,
+                    (bf16*)w_lo, (int)J, (int)K, Jpad);
 }
 
 // groups > 0: `labels` are first reduced from that many column groups of `partial` (see assign_tc.cu).
