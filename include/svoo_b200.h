@@ -38,7 +38,7 @@ enum {
   SVOO_ERR_WORKSPACE = -4,   /* workspace too small (see *_workspace_bytes)      */
   SVOO_ERR_ALIGN = -5,       /* a tensor pointer is not 16-byte aligned          */
   SVOO_ERR_CLUSTERS = -6,    /* cluster count above SVOO_MAX_CLUSTERS            */
-  SVOO_ERR_STATIC_SCRATCH = -7 /* problem too large for the built-in scratch array */
+  SVOO_ERR_STATIC_SCRATCH = -7 /* BH * ceil(N / 2048) * K above the limit of svoo_b200_sort_labels_static */
 };
 
 #define SVOO_MAX_CLUSTERS 1024   /* per side; the reference ships QC=256, KC=1024 */
@@ -74,6 +74,18 @@ int svoo_b200_workspace_bytes(int64_t BH, int64_t N, int64_t QC, int64_t KC, int
 int svoo_b200_cocluster(const void* q, const void* k,
                         const int32_t* q_init_idx, const int32_t* k_init_idx,
                         int64_t BH, int64_t N, int64_t D, int64_t QC, int64_t KC, int32_t iters,
+                        int32_t* qlabels, int32_t* klabels,
+                        void* qcentroids, void* kcentroids,
+                        int32_t* qsizes, int32_t* ksizes,
+                        int32_t* q_sorted_idx, int32_t* q_offsets,
+                        int32_t* k_sorted_idx, int32_t* k_offsets,
+                        void* workspace, int64_t workspace_bytes, void* stream);
+
+/* The same on the first N rows of every head of q and k [BH, head_rows, 128], head_rows >= N (a joint-attention
+ * layer: video rows first, text rows behind them, which are not clustered). */
+int svoo_b200_cocluster_rows(const void* q, const void* k,
+                        const int32_t* q_init_idx, const int32_t* k_init_idx,
+                        int64_t BH, int64_t N, int64_t head_rows, int64_t D, int64_t QC, int64_t KC, int32_t iters,
                         int32_t* qlabels, int32_t* klabels,
                         void* qcentroids, void* kcentroids,
                         int32_t* qsizes, int32_t* ksizes,

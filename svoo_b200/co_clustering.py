@@ -20,6 +20,14 @@ def _as_bf16(x: torch.Tensor) -> torch.Tensor:
     return x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
 
 
+def _cluster_inputs(q: torch.Tensor, k: torch.Tensor):
+    """q and k as the clustering reads them: bf16, in place where their rows allow it, else copied."""
+    q, k = _as_bf16(q), _as_bf16(k)
+    if ops.rows_in_place(q) and ops.rows_in_place(k) and (q.shape[0] == 1 or q.stride(0) == k.stride(0)):
+        return q, k
+    return q.contiguous(), k.contiguous()
+
+
 def draw_init_indices(BH: int, N: int, num_q: int, num_k: int, device, generator=None):
     """Initial centroid token indices in the reference's draw order: q first, then k
     (svoo/co_clustering.py:2417-2421)."""
@@ -36,16 +44,16 @@ def co_cluster(q_flat: torch.Tensor, k_flat: torch.Tensor, num_q_centroids: int,
     reference always draws, svoo/models/wan/attention.py:641-647)."""
     assert q_flat.is_cuda and k_flat.is_cuda, "tensors must be on CUDA"
     BH, N, D = q_flat.shape
+    q_in, k_in = _cluster_inputs(q_flat, k_flat)
     if init_centroids is not None:
         qc0, kc0 = init_centroids
-        return ops.cocluster(_as_bf16(q_flat).contiguous(), _as_bf16(k_flat).contiguous(), None, None, max_iters,
+        return ops.cocluster(q_in, k_in, None, None, max_iters,
                              init_centroids=(_as_bf16(qc0).contiguous(), _as_bf16(kc0).contiguous()))
     if init_indices is None:
         init_indices = draw_init_indices(BH, N, num_q_centroids, num_k_centroids, q_flat.device, generator)
     q_idx, k_idx = init_indices
     assert q_idx.shape == (BH, num_q_centroids) and k_idx.shape == (BH, num_k_centroids)
-    return ops.cocluster(_as_bf16(q_flat).contiguous(), _as_bf16(k_flat).contiguous(),
-                         q_idx.to(q_flat.device), k_idx.to(q_flat.device), max_iters)
+    return ops.cocluster(q_in, k_in, q_idx.to(q_flat.device), k_idx.to(q_flat.device), max_iters)
 
 
 def co_cluster_tokens(q_flat, k_flat, num_q_centroids, num_k_centroids, max_iters=10, *, init_indices=None,

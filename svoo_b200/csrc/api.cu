@@ -3,13 +3,13 @@
 #include "common.cuh"
 
 namespace svoo {
-cudaError_t launch_gather_rows(const void*, const int32_t*, void*, int64_t, int64_t, int64_t, cudaStream_t);
+cudaError_t launch_gather_rows(const void*, int64_t, const int32_t*, void*, int64_t, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_prologue(const void*, const void*, void*, void*, int64_t, int64_t, int64_t, cudaStream_t);
-cudaError_t launch_assign_tc(const void*, const void*, const void*, int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
+cudaError_t launch_assign_tc(const void*, int64_t, const void*, const void*, int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
 int assign_groups(int64_t J);
 cudaError_t launch_assign_reduce(const int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_sort_labels(const int2*, int, int32_t*, int64_t, int64_t, int64_t, int32_t*, int32_t*, int32_t*, cudaStream_t);
-cudaError_t launch_centroid_update(const void*, const int32_t*, const int32_t*, const void*, void*, int32_t*, float*,
+cudaError_t launch_centroid_update(const void*, int64_t, const int32_t*, const int32_t*, const void*, void*, int32_t*, float*,
                                    int64_t, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_offsets_from_sizes(const int32_t*, int32_t*, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_permute(const void*, const int32_t*, void*, int64_t, int64_t, int64_t, int64_t, bool, cudaStream_t);
@@ -127,7 +127,7 @@ int svoo_b200_cocluster_assign(const void* x, const void* form_centroids, const 
                             ws_at<void>(workspace, w.w_lo), BH, J, K, st));
   SVOO_CUDA(cudaMemsetAsync(ws_at<int32_t>(workspace, w.status) + 1, 0, 4, st));
   int2* partial = ws_at<int2>(workspace, w.assign_partial);
-  SVOO_CUDA(launch_assign_tc(x, ws_at<void>(workspace, w.w_hi), ws_at<void>(workspace, w.w_lo), partial,
+  SVOO_CUDA(launch_assign_tc(x, N, ws_at<void>(workspace, w.w_hi), ws_at<void>(workspace, w.w_lo), partial,
                              ws_at<int32_t>(workspace, w.status) + 1, BH, N, J, st));
   SVOO_CUDA(launch_assign_reduce(partial, labels, BH, N, J, st));
   return SVOO_OK;
@@ -172,13 +172,13 @@ int svoo_b200_centroid_update(const void* x, const int32_t* sorted_idx, const in
   if (!aligned16(x)) return SVOO_ERR_ALIGN;
   const Workspace w = workspace_layout(BH, N, K, K);
   if (workspace_bytes < w.total) return SVOO_ERR_WORKSPACE;
-  SVOO_CUDA(launch_centroid_update(x, sorted_idx, offsets, old_centroids, new_centroids, sizes,
+  SVOO_CUDA(launch_centroid_update(x, N, sorted_idx, offsets, old_centroids, new_centroids, sizes,
                                    ws_at<float>(workspace, w.partial), BH, N, K, (cudaStream_t)stream));
   return SVOO_OK;
 }
 
-int svoo_b200_cocluster(const void* q, const void* k, const int32_t* q_init_idx, const int32_t* k_init_idx, int64_t BH,
-                        int64_t N, int64_t D, int64_t QC, int64_t KC, int32_t iters, int32_t* qlabels,
+int svoo_b200_cocluster_rows(const void* q, const void* k, const int32_t* q_init_idx, const int32_t* k_init_idx, int64_t BH,
+                             int64_t N, int64_t head_rows, int64_t D, int64_t QC, int64_t KC, int32_t iters, int32_t* qlabels,
                         int32_t* klabels, void* qcentroids, void* kcentroids, int32_t* qsizes, int32_t* ksizes,
                         int32_t* q_sorted_idx, int32_t* q_offsets, int32_t* k_sorted_idx, int32_t* k_offsets,
                         void* workspace, int64_t workspace_bytes, void* stream) {
@@ -187,6 +187,8 @@ int svoo_b200_cocluster(const void* q, const void* k, const int32_t* q_init_idx,
     return SVOO_ERR_NULL;
   if ((q_init_idx == nullptr) != (k_init_idx == nullptr)) return SVOO_ERR_NULL;   // both (fresh start) or neither (warm start)
   SVOO_TRY(check_tokens(BH, N, D));
+  if (head_rows < N) return SVOO_ERR_SHAPE;
+  SVOO_TRY(check_tokens(BH, head_rows, D));
   SVOO_TRY(check_clusters(QC));
   SVOO_TRY(check_clusters(KC));
   if (iters < 1 || iters > 1000) return SVOO_ERR_SHAPE;
@@ -203,22 +205,32 @@ int svoo_b200_cocluster(const void* q, const void* k, const int32_t* q_init_idx,
 
   SVOO_CUDA(cudaMemsetAsync(status, 0, 4, st));
   if (q_init_idx) {
-    SVOO_CUDA(launch_gather_rows(q, q_init_idx, qcentroids, BH, N, QC, st));
-    SVOO_CUDA(launch_gather_rows(k, k_init_idx, kcentroids, BH, N, KC, st));
+    SVOO_CUDA(launch_gather_rows(q, head_rows, q_init_idx, qcentroids, BH, N, QC, st));
+    SVOO_CUDA(launch_gather_rows(k, head_rows, k_init_idx, kcentroids, BH, N, KC, st));
   }
   for (int it = 0; it < iters; ++it) {
     // keys: profile over the query centroids
     SVOO_CUDA(launch_prologue(kcentroids, qcentroids, w_hi, w_lo, BH, KC, QC, st));
-    SVOO_CUDA(launch_assign_tc(k, w_hi, w_lo, apart, status, BH, N, KC, st));
+    SVOO_CUDA(launch_assign_tc(k, head_rows, w_hi, w_lo, apart, status, BH, N, KC, st));
     SVOO_CUDA(launch_sort_labels(apart, assign_groups(KC), klabels, BH, N, KC, k_sorted_idx, k_offsets, nullptr, st));
-    SVOO_CUDA(launch_centroid_update(k, k_sorted_idx, k_offsets, kcentroids, kcentroids, ksizes, partial, BH, N, KC, st));
+    SVOO_CUDA(launch_centroid_update(k, head_rows, k_sorted_idx, k_offsets, kcentroids, kcentroids, ksizes, partial, BH, N, KC, st));
     // queries: profile over the just-updated key centroids
     SVOO_CUDA(launch_prologue(qcentroids, kcentroids, w_hi, w_lo, BH, QC, KC, st));
-    SVOO_CUDA(launch_assign_tc(q, w_hi, w_lo, apart, status, BH, N, QC, st));
+    SVOO_CUDA(launch_assign_tc(q, head_rows, w_hi, w_lo, apart, status, BH, N, QC, st));
     SVOO_CUDA(launch_sort_labels(apart, assign_groups(QC), qlabels, BH, N, QC, q_sorted_idx, q_offsets, nullptr, st));
-    SVOO_CUDA(launch_centroid_update(q, q_sorted_idx, q_offsets, qcentroids, qcentroids, qsizes, partial, BH, N, QC, st));
+    SVOO_CUDA(launch_centroid_update(q, head_rows, q_sorted_idx, q_offsets, qcentroids, qcentroids, qsizes, partial, BH, N, QC, st));
   }
   return SVOO_OK;
+}
+
+int svoo_b200_cocluster(const void* q, const void* k, const int32_t* q_init_idx, const int32_t* k_init_idx, int64_t BH,
+                        int64_t N, int64_t D, int64_t QC, int64_t KC, int32_t iters, int32_t* qlabels,
+                        int32_t* klabels, void* qcentroids, void* kcentroids, int32_t* qsizes, int32_t* ksizes,
+                        int32_t* q_sorted_idx, int32_t* q_offsets, int32_t* k_sorted_idx, int32_t* k_offsets,
+                        void* workspace, int64_t workspace_bytes, void* stream) {
+  return svoo_b200_cocluster_rows(q, k, q_init_idx, k_init_idx, BH, N, N, D, QC, KC, iters, qlabels, klabels, qcentroids,
+                                  kcentroids, qsizes, ksizes, q_sorted_idx, q_offsets, k_sorted_idx, k_offsets, workspace,
+                                  workspace_bytes, stream);
 }
 
 int svoo_b200_permute(const void* x, const int32_t* sorted_idx, int64_t BH, int64_t N, int64_t D,
@@ -687,22 +699,11 @@ int svoo_b200_layer(const void* q, const void* k, const void* v, const int32_t* 
   int32_t* ksorted = static_cast<int32_t*>(at(l.ksorted));
   int32_t* qoff = static_cast<int32_t*>(at(l.qoff));
   int32_t* koff = static_cast<int32_t*>(at(l.koff));
-  const void* qv = q;
-  const void* kv = k;
-  if (text > 0) {
-    // the clustering reads dense [BH, N, 128] video rows: stage them where the permuted Q and K
-    // will be written once the clustering is done
-    SVOO_CUDA(cudaMemcpy2DAsync(at(l.qp), (size_t)N * kRowBytes, q, (size_t)S * kRowBytes, (size_t)N * kRowBytes, (size_t)BH,
-                                cudaMemcpyDeviceToDevice, st));
-    SVOO_CUDA(cudaMemcpy2DAsync(at(l.kp), (size_t)N * kRowBytes, k, (size_t)S * kRowBytes, (size_t)N * kRowBytes, (size_t)BH,
-                                cudaMemcpyDeviceToDevice, st));
-    qv = at(l.qp);
-    kv = at(l.kp);
-  }
-  SVOO_TRY(svoo_b200_cocluster(qv, kv, q_init_idx, k_init_idx, BH, N, D, QC, KC, iters, static_cast<int32_t*>(at(l.qlabels)),
-                               static_cast<int32_t*>(at(l.klabels)), at(l.qcent), at(l.kcent),
-                               static_cast<int32_t*>(at(l.qsizes)), static_cast<int32_t*>(at(l.ksizes)), qsorted, qoff,
-                               ksorted, koff, workspace, workspace_bytes, stream));
+  // the clustering reads the N video rows of every head in place
+  SVOO_TRY(svoo_b200_cocluster_rows(q, k, q_init_idx, k_init_idx, BH, N, S, D, QC, KC, iters, static_cast<int32_t*>(at(l.qlabels)),
+                                    static_cast<int32_t*>(at(l.klabels)), at(l.qcent), at(l.kcent),
+                                    static_cast<int32_t*>(at(l.qsizes)), static_cast<int32_t*>(at(l.ksizes)), qsorted, qoff,
+                                    ksorted, koff, workspace, workspace_bytes, stream));
   uint8_t* map = static_cast<uint8_t*>(at(l.map));
   if (top_p >= 1.0f) {
     SVOO_CUDA(cudaMemsetAsync(map, 1, (size_t)(BH * QC * KC), st));

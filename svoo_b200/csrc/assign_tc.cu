@@ -134,7 +134,7 @@ template <int JB, bool kEuclid>
 __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
     const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_hi,
     const __grid_constant__ CUtensorMap tm_lo, int2* __restrict__ partial, int BH, int N, int J, int w_head_rows,
-    const float* __restrict__ bias, int32_t* __restrict__ status) {
+    int x_head_rows, const float* __restrict__ bias, int32_t* __restrict__ status) {
   using C = AsgCfg<JB>;
   constexpr int NS = C::kXStages;
   constexpr uint32_t kIdesc = idesc_bf16(128, JB, false);
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kAsgThreads, 1) assign_tc_kernel(
         if (!mbar_wait(bar(C::X_EMPTY + s), ((i / NS) & 1) ^ 1, abort_flag)) break;
         mbar_expect_tx(bar(C::X_FULL + s), kAsgXBytes);
         for (int h = 0; h < 2; ++h)
-          tma_load_2d(x_s + s * kAsgXBytes + h * kAsgXHalf, &tm_x, h * 64, job.bh * N + job.t * kAsgXT, bar(C::X_FULL + s));
+          tma_load_2d(x_s + s * kAsgXBytes + h * kAsgXHalf, &tm_x, h * 64, job.bh * x_head_rows + job.t * kAsgXT, bar(C::X_FULL + s));
       }
     }
   } else if (warp == 1) {
@@ -355,12 +355,12 @@ bool make_row_tensor_map(CUtensorMap* map, const void* ptr, int64_t rows, int bo
 }  // namespace tc
 
 template <int JB, bool kEuclid>
-static cudaError_t launch_assign_tc_jb(const void* x, const void* w_hi, const void* w_lo, const float* bias, int2* partial,
+static cudaError_t launch_assign_tc_jb(const void* x, int64_t x_head_rows, const void* w_hi, const void* w_lo, const float* bias, int2* partial,
                                        int32_t* status, int64_t BH, int64_t N, int64_t J, int w_head_rows,
                                        cudaStream_t st) {
   using C = tc::AsgCfg<JB>;
   alignas(64) CUtensorMap mx, mh, ml;
-  if (!tc::make_row_tensor_map(&mx, x, BH * N, tc::kAsgXT) || !tc::make_row_tensor_map(&mh, w_hi, BH * w_head_rows, JB) ||
+  if (!tc::make_row_tensor_map(&mx, x, (BH - 1) * x_head_rows + N, tc::kAsgXT) || !tc::make_row_tensor_map(&mh, w_hi, BH * w_head_rows, JB) ||
       !tc::make_row_tensor_map(&ml, w_lo, BH * w_head_rows, JB))
     return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(tc::assign_tc_kernel<JB, kEuclid>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -372,7 +372,7 @@ static cudaError_t launch_assign_tc_jb(const void* x, const void* w_hi, const vo
   const int64_t total = BH * ceil_div64(J, JB) * ceil_div64(N, tc::kAsgXT);
   const unsigned grid = (unsigned)(total < sms ? total : sms);
   return launch_pdl(tc::assign_tc_kernel<JB, kEuclid>, dim3(grid), dim3(tc::kAsgThreads), (size_t)C::kSmemBytes, st, mx, mh, ml,
-                    partial, (int)BH, (int)N, (int)J, w_head_rows, bias, status);
+                    partial, (int)BH, (int)N, (int)J, w_head_rows, (int)x_head_rows, bias, status);
 }
 
 // Column groups per token in `partial`: two per W block.
@@ -385,12 +385,12 @@ cudaError_t launch_assign_reduce(const int2* partial, int32_t* labels, int64_t B
 }
 
 // Leaves the winners of the column groups in `partial`; the label sort or launch_assign_reduce reads them.
-cudaError_t launch_assign_tc(const void* x, const void* w_hi, const void* w_lo, int2* partial, int32_t* status, int64_t BH,
+cudaError_t launch_assign_tc(const void* x, int64_t x_head_rows, const void* w_hi, const void* w_lo, int2* partial, int32_t* status, int64_t BH,
                              int64_t N, int64_t J, cudaStream_t st) {
   const int Jpad = pad_clusters(J);
   count_launches(1);
-  return J <= 128 ? launch_assign_tc_jb<128, false>(x, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st)
-                  : launch_assign_tc_jb<256, false>(x, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st);
+  return J <= 128 ? launch_assign_tc_jb<128, false>(x, x_head_rows, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st)
+                  : launch_assign_tc_jb<256, false>(x, x_head_rows, w_hi, w_lo, nullptr, partial, status, BH, N, J, Jpad, st);
 }
 
 // bias[bh, j] = -sum_d bf16(c_d * c_d) / 2: the centroid term of the squared distance with the
@@ -423,8 +423,8 @@ cudaError_t launch_euclid_assign_tc(const void* x, const void* centroids, float*
                              (const bf16*)centroids, bias, BH * K);
   if (e != cudaSuccess) return e;
   count_launches(2);
-  return K <= 128 ? launch_assign_tc_jb<128, true>(x, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st)
-                  : launch_assign_tc_jb<256, true>(x, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st);
+  return K <= 128 ? launch_assign_tc_jb<128, true>(x, N, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st)
+                  : launch_assign_tc_jb<256, true>(x, N, centroids, centroids, bias, partial, status, BH, N, K, (int)K, st);
 }
 
 }  // namespace svoo

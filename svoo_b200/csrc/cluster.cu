@@ -18,7 +18,7 @@ namespace svoo {
 // centroids[bh,c,:] = x[bh, idx[bh,c], :]     (svoo/co_clustering.py:2417-2421)
 // ---------------------------------------------------------------------------------------
 __global__ void gather_rows_kernel(const bf16* __restrict__ x, const int32_t* __restrict__ idx,
-                                   bf16* __restrict__ out, int N, int K) {
+                                   bf16* __restrict__ out, int N, int K, int64_t x_head_rows) {
   pdl_trigger();
   pdl_wait();
   const int bh = blockIdx.y;
@@ -27,7 +27,7 @@ __global__ void gather_rows_kernel(const bf16* __restrict__ x, const int32_t* __
   const int lane = threadIdx.x % 16;
   int src = idx[(int64_t)bh * K + c];
   src = min(max(src, 0), N - 1);
-  const uint4* s = reinterpret_cast<const uint4*>(x + ((int64_t)bh * N + src) * kHeadDim);
+  const uint4* s = reinterpret_cast<const uint4*>(x + (bh * x_head_rows + src) * kHeadDim);
   uint4* d = reinterpret_cast<uint4*>(out + ((int64_t)bh * K + c) * kHeadDim);
   d[lane] = s[lane];
 }
@@ -406,7 +406,8 @@ __device__ __forceinline__ void slab_range(int begin, int end, int z, int nslabs
 __global__ void __launch_bounds__(256) centroid_partial_kernel(const bf16* __restrict__ x,
                                                                const int32_t* __restrict__ sorted_idx,
                                                                const int32_t* __restrict__ offsets,
-                                                               float* __restrict__ partial, int N, int K, int nslabs) {
+                                                               float* __restrict__ partial, int N, int K, int nslabs,
+                                                               int64_t x_head_rows) {
   __shared__ float red[16][kHeadDim + 4];
   pdl_trigger();
   pdl_wait();
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(256) centroid_partial_kernel(const bf16* __res
   if (s0 >= s1) return;
   const int grp = threadIdx.x / 16, lane = threadIdx.x % 16;
   const int32_t* idx = sorted_idx + (int64_t)bh * N;
-  const bf16* xb = x + (int64_t)bh * N * kHeadDim;
+  const bf16* xb = x + bh * x_head_rows * kHeadDim;
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -520,11 +521,12 @@ __global__ void __launch_bounds__(1024) offsets_from_sizes_kernel(const int32_t*
 // ---------------------------------------------------------------------------------------
 // Host launchers (called from api.cu)
 // ---------------------------------------------------------------------------------------
-cudaError_t launch_gather_rows(const void* x, const int32_t* idx, void* out, int64_t BH, int64_t N, int64_t K,
-                               cudaStream_t st) {
+// x_head_rows >= N: rows from one head of x to the next.
+cudaError_t launch_gather_rows(const void* x, int64_t x_head_rows, const int32_t* idx, void* out, int64_t BH, int64_t N,
+                               int64_t K, cudaStream_t st) {
   dim3 grid((unsigned)ceil_div64(K, 16), (unsigned)BH);
   count_launches(1);
-  return launch_pdl(gather_rows_kernel, grid, dim3(256), 0, st, (const bf16*)x, idx, (bf16*)out, (int)N, (int)K);
+  return launch_pdl(gather_rows_kernel, grid, dim3(256), 0, st, (const bf16*)x, idx, (bf16*)out, (int)N, (int)K, x_head_rows);
 }
 
 cudaError_t launch_prologue(const void* own, const void* form, void* w_hi, void* w_lo, int64_t BH, int64_t J,
@@ -581,7 +583,7 @@ cudaError_t launch_sort_labels(const int2* partial, int groups, int32_t* labels,
   return cudaLaunchKernelEx(&cfg, kernel, partial, labels, sorted_idx, offsets, sizes, (int)BH, (int)N, (int)K);
 }
 
-cudaError_t launch_centroid_update(const void* x, const int32_t* sorted_idx, const int32_t* offsets,
+cudaError_t launch_centroid_update(const void* x, int64_t x_head_rows, const int32_t* sorted_idx, const int32_t* offsets,
                                    const void* old_c, void* new_c, int32_t* sizes, float* partial, int64_t BH,
                                    int64_t N, int64_t K, cudaStream_t st) {
   // slabs per cluster: enough for clusters of four times the mean size to keep the 256-row minimum,
@@ -591,7 +593,7 @@ cudaError_t launch_centroid_update(const void* x, const int32_t* sorted_idx, con
   nslabs = nslabs < 1 ? 1 : (nslabs > kCentroidSlabs ? kCentroidSlabs : nslabs);
   dim3 grid((unsigned)K, (unsigned)nslabs, (unsigned)BH);
   cudaError_t e = launch_pdl(centroid_partial_kernel, grid, dim3(256), 0, st, (const bf16*)x, sorted_idx, offsets, partial,
-                             (int)N, (int)K, nslabs);
+                             (int)N, (int)K, nslabs, x_head_rows);
   if (e != cudaSuccess) return e;
   dim3 grid2((unsigned)ceil_div64(K, kFinalizePerCta), (unsigned)BH);
   count_launches(2);

@@ -67,12 +67,9 @@ def sparse_attention_layer(query: torch.Tensor, key: torch.Tensor, value: torch.
     mark("start")
     c = clustering
     if c is None:
-        if context_length:
-            qv, kv = q[:, :n_video].contiguous(), k[:, :n_video].contiguous()
-        else:
-            qv, kv = q.contiguous(), k.contiguous()
-        c = cc.co_cluster(qv, kv, num_q_centroids, num_k_centroids, kmeans_iters, init_indices=init_indices)
-        del qv, kv
+        # the video rows of every head, read in place
+        c = cc.co_cluster(q[:, :n_video], k[:, :n_video], num_q_centroids, num_k_centroids, kmeans_iters,
+                          init_indices=init_indices)
     mark("cocluster")
     if ear_gamma is not None:
         return _ear_layer(q, k, v, c, top_p, min_kc_ratio, float(ear_gamma), context_length, peer_out, value_ready, mark,

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import functools
 from typing import Dict, Optional, Sequence, Tuple
 
 import torch
@@ -33,6 +34,15 @@ def _tokens(x: torch.Tensor) -> Tuple[int, int, int]:
     if x.dim() != 3 or x.dtype != torch.bfloat16:
         raise ValueError(f"expected bf16 [BH, N, {HEAD_DIM}] tokens, got {x.dtype} {tuple(x.shape)}")
     return x.shape
+
+
+def rows_in_place(x: torch.Tensor) -> bool:
+    """Whether the clustering can read x [BH, N, 128] where it is: CUDA, dense rows, heads a whole number
+    (>= N) of rows apart -- a tensor of its own or the leading rows of longer per-head sequences."""
+    return (x.is_cuda and x.dim() == 3 and x.shape[-1] == HEAD_DIM and x.stride(-1) == 1 and
+            (x.shape[1] == 1 or x.stride(1) == HEAD_DIM) and x.data_ptr() % 16 == 0 and
+            (x.shape[0] == 1 or (x.stride(0) % HEAD_DIM == 0 and x.stride(0) >= x.shape[1] * HEAD_DIM and
+                                 x.shape[0] * x.stride(0) // HEAD_DIM < 2 ** 31 and x.stride(0) // HEAD_DIM <= 1 << 24)))
 
 
 def workspace_bytes(BH: int, N: int, QC: int, KC: int) -> int:
@@ -71,11 +81,14 @@ def cocluster(q: torch.Tensor, k: torch.Tensor, q_init_idx: Optional[torch.Tenso
               k_init_idx: Optional[torch.Tensor], iters: int,
               init_centroids: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> Clustering:
     """Co-clustering from initial centroid token indices, or (warm start) from `init_centroids` =
-    (q centroids [BH,QC,128], k centroids [BH,KC,128]), which are not modified."""
-    _need_cuda(q, k)
+    (q centroids [BH,QC,128], k centroids [BH,KC,128]), which are not modified.  q and k may be the leading
+    rows of longer per-head sequences (rows_in_place), spaced alike."""
+    if not (rows_in_place(q) and rows_in_place(k) and (q.shape[0] == 1 or q.stride(0) == k.stride(0))):
+        _need_cuda(q, k)
     BH, N, D = _tokens(q)
     if k.shape != q.shape or k.dtype != q.dtype:
         raise ValueError("q and k must have the same shape and dtype")
+    head_rows = N if BH == 1 else q.stride(0) // HEAD_DIM
     dev = q.device
     i32 = dict(dtype=torch.int32, device=dev)
     if init_centroids is not None:
@@ -102,8 +115,8 @@ def cocluster(q: torch.Tensor, k: torch.Tensor, q_init_idx: Optional[torch.Tenso
         torch.empty(BH, N, **i32), torch.empty(BH, N, **i32),
         torch.empty(BH, QC + 1, **i32), torch.empty(BH, KC + 1, **i32))
     ws = workspace(dev, BH, N, QC, KC)
-    check(LIB.svoo_b200_cocluster(
-        q.data_ptr(), k.data_ptr(), qi_ptr, ki_ptr, BH, N, D, QC, KC, int(iters),
+    check(LIB.svoo_b200_cocluster_rows(
+        q.data_ptr(), k.data_ptr(), qi_ptr, ki_ptr, BH, N, head_rows, D, QC, KC, int(iters),
         c.qlabels.data_ptr(), c.klabels.data_ptr(), c.qcentroids.data_ptr(), c.kcentroids.data_ptr(),
         c.qsizes.data_ptr(), c.ksizes.data_ptr(), c.q_sorted_idx.data_ptr(), c.q_offsets.data_ptr(),
         c.k_sorted_idx.data_ptr(), c.k_offsets.data_ptr(), ws.data_ptr(), ws.numel(), _stream()), "cocluster")
@@ -290,6 +303,18 @@ def sparse_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, block_map_u8:
         raise ValueError("the log-sum-exp output needs the tcgen05 kernel")
     check(LIB.svoo_b200_sparse_attn_simt(*head, ridx, ws.data_ptr(), ws.numel(), _stream()), "sparse_attn")
     return y
+
+
+@functools.lru_cache(maxsize=None)
+def _all_heads(H: int):
+    return (ctypes.c_int32 * H)(*range(H))
+
+
+def token_major(out: torch.Tensor):
+    """`peer_out` for sparse_attn / sparse_attn_ear that stores the rows of all H <= 128 heads into the local
+    tensor out [1, S, H, 128]."""
+    _, S, H, _ = out.shape
+    return (ctypes.c_void_p * 1)(out.data_ptr()), _all_heads(H), 1, S, H
 
 
 def attention_status(device: torch.device, BH: int, S: int, QC: int, KC: int) -> int:

@@ -165,19 +165,24 @@ class _SAPBase:
     def _sparse(self, query, key, value, prompt_length=None):
         cfg, H, S, D = query.shape
         n_video = self.num_frame * self.frame_size
-        if self.context_length:
-            qv, kv = query[:, :, :n_video].contiguous(), key[:, :, :n_video].contiguous()
-        else:
-            qv, kv = query, key
+        qv, kv = (query[:, :, :n_video], key[:, :, :n_video]) if self.context_length else (query, key)
         c = self.kmeans_clustering(qv, kv, self.layer_idx)
         extra = 2 if self.context_length else 0
         self._last_shape = (query.device, cfg * H, S, n_video, self.num_q_centroids + extra, self.num_k_centroids + extra)
         ratio = self._get_min_kc_ratio_for_heads_from_step(self.current_inference_step, H)
+        # the attention stores its rows token-major, so that the callers' transpose(1, 2).flatten(2, 3) is a view
+        rows, peer_out = None, None
+        if cfg == 1 and H <= 128:
+            rows = torch.empty(cfg, S, H, D, dtype=query.dtype, device=query.device)
+            peer_out = ops.token_major(rows)
         out, state = sparse_attention_layer(query, key, value, num_q_centroids=self.num_q_centroids,
                                             num_k_centroids=self.num_k_centroids, kmeans_iters=0,
                                             top_p=self.top_p_kmeans, min_kc_ratio=ratio, clustering=c,
                                             context_length=self.context_length, prompt_length=prompt_length,
-                                            return_state=True, ear_gamma=self.ear_gamma if self.use_ear else None)
+                                            return_state=True, ear_gamma=self.ear_gamma if self.use_ear else None,
+                                            peer_out=peer_out)
+        if peer_out is not None:
+            out = rows.transpose(1, 2)
         self.last_block_map = state.block_map              # uint8 [H, QC(+2), KC(+2)] of the last sparse call
         return out
 
