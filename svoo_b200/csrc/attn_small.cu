@@ -311,6 +311,8 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
     }
   }
   // ------------------------------------------------------------------ teardown
+  // Q was requested before the number of keys was known; without keys nobody has waited for it.
+  if (tid == 0) mbar_drain(bar(SM_Q_FULL), 0);
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && *abort_flag) atomicExch(status, 1);

@@ -91,3 +91,28 @@ def test_attention_tile_edges(name, ear):
     again = ops.sparse_attn(q, k, v, m, q_off, k_off, out_row_idx=perm) if not ear else \
         ops.sparse_attn_ear(q, k_ext, v_ext, m, q_off, k_off, out_row_idx=perm)
     assert torch.equal(again, got)
+
+
+@pytest.mark.parametrize("rows", [1, 64, 65, 128])
+def test_query_clusters_without_keys(rows):
+    """Most query clusters have no keys: their CTAs end at once and others start in their place.  Zero rows for them,
+    the others undisturbed."""
+    from svoo_b200 import ops
+    dev = torch.device("cuda")
+    H, QC, KC = 8, 160, 24
+    gen = torch.Generator().manual_seed(rows)
+    S = rows * QC
+    qs = torch.full((H, QC), rows)
+    ks = torch.full((H, KC), S // KC)
+    ks[:, -1] += S - ks[0].sum()
+    q, k, v = (torch.randn(H, S, 128, generator=gen).to(dev, torch.bfloat16) for _ in range(3))
+    sel = torch.zeros(H, QC, KC, dtype=torch.bool)
+    sel[:, ::5, 3] = True
+    sel[:, 2::5, ::7] = True
+    q_off, k_off = _offsets(qs, dev), _offsets(ks, dev)
+    got = ops.sparse_attn(q, k, v, sel.to(torch.uint8).to(dev), q_off, k_off)
+    assert ops.attention_status(dev, H, S, QC, KC) == 0
+    dead = torch.repeat_interleave(~sel.any(-1), rows, dim=1).to(dev)
+    assert (got[dead] == 0).all()
+    want = _reference(q[:1], k[:1], v[:1], sel[:1], qs[:1], ks[:1], 128 ** -0.5)
+    assert (got[:1].float() - want).abs().max() <= 2.5 * 2.0 ** -9 * v.float().abs().max()
