@@ -39,7 +39,7 @@ struct SmallSmem {
 static_assert(2 * (SmallSmem<true>::kBytes + 1024) <= 228 * 1024, "two CTAs share an SM");
 
 // PV_DONE has one barrier per step parity because the softmax does not wait for every PV: when it asks
-// for step j, step j - 2 is known to be complete (S of step j was issued behind it) but step j - 1 is not.
+// for step j, step j - 2 is known to be complete (S of step j was issued after it) but step j - 1 is not.
 enum SmBar { SM_Q_FULL = 0, SM_K_FULL = 1, SM_K_EMPTY = 3, SM_V_FULL = 5, SM_V_EMPTY = 7, SM_S_FULL = 9, SM_P_READY = 11,
              SM_PV_DONE = 13, SM_NUM_BARS = 15 };
 // TMEM columns: two S buffers (P of a step overwrites the first half of its S buffer), then O.
@@ -163,8 +163,9 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
     if (pending) report((T - 1) & 1);
   } else if (warp == kSmMmaWarp) {
     // ---------------------------------------------------------------- MMA issuer
-    // The MMAs of one thread execute in order, so QK of step j + 2 may overwrite the S buffer that holds
-    // P of step j once it is issued behind the PV that reads it.
+    // QK of step j + 2 overwrites the S buffer that holds P of step j, so it is issued when the PV that reads
+    // that P has completed: the order of two MMAs is only promised for one accumulator and shape.  The
+    // softmax is at work on step j + 1 meanwhile, and the other CTA of the SM on its own steps.
     if (lane == 0 && T > 0) {
       constexpr uint32_t kDescHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
       const uint32_t q_lo = ((q_s & 0x3FFFFu) >> 4) | (1u << 16);
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
                      (j > 0 || ks > 0) ? 1u : 0u);
         tc_commit(bar(SM_V_EMPTY + st));
         tc_commit(bar(SM_PV_DONE + st));
-        if (j + 2 < T) ok = qk(j + 2);
+        if (j + 2 < T) ok = mbar_wait(bar(SM_PV_DONE + st), (j >> 1) & 1, abort_flag) && qk(j + 2);
       }
     }
   } else {
