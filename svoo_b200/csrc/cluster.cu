@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
     }
     tot[k] = run;
   }
+  __syncwarp();                                          // the lanes left the loop at different counts; the barrier is .aligned
   cluster_arrive();
   cluster_wait();
 
@@ -331,6 +332,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
       }
     sum += all[u];
   }
+  __syncwarp();
   cluster_arrive();                                      // this CTA has read the others' totals (waited for at the end)
   int incl = sum;
 #pragma unroll
@@ -386,6 +388,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
       }
     }
   }
+  __syncwarp();
   cluster_wait();
 }
 

@@ -36,3 +36,15 @@ def test_sort_reduces_the_assignment_winners(J):
     assert torch.equal(c.klabels, klab)
     assert torch.equal(c.k_sorted_idx.long(), torch.argsort(klab, dim=1, stable=True))
     assert torch.equal(c.ksizes.long(), torch.stack([torch.bincount(r, minlength=J) for r in klab.long()]))
+
+
+@pytest.mark.parametrize("K", [1, 31, 33, 500, 511, 513, 1023])
+def test_sort_of_sixteen_ctas_with_partial_warps(K):
+    """Sixteen CTAs per head with cluster counts that end inside a warp: its lanes meet the cluster barriers from
+    loops of different lengths."""
+    from svoo_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    lab = torch.randint(0, K, (3, 40003), generator=gen, device="cuda", dtype=torch.int32)
+    idx, off = ops.sort_labels(lab, K)
+    assert torch.equal(idx.long(), torch.argsort(lab, dim=1, stable=True))
+    assert torch.equal(off[:, 1:].long(), torch.stack([torch.bincount(r, minlength=K) for r in lab.long()]).cumsum(1))
