@@ -348,14 +348,10 @@ __device__ void build_runs(const uint8_t* __restrict__ map, const int32_t* __res
   const int r = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t row = (int64_t)bh * QC + min(i0 + r, QC - 1);
   const uint8_t* m = map + row * KC;
-  // bytes [32 lane, 32 lane + 32) of the row as nine aligned words, of which only those that hold one of them are read
-  const int j0 = lane * 32, bytes = max(min(KC - j0, 32), 0);
-  const uintptr_t at = reinterpret_cast<uintptr_t>(m + j0);
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
-  const int skew = (int)(at & 3);
+  // bytes [32 lane, 32 lane + 32) of the row
+  const int j0 = lane * 32;
   uint32_t w[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) w[i] = 4 * i < bytes + skew && bytes > 0 ? __ldg(words + i) : 0;
+  const int skew = map_words(w, m + j0, max(min(KC - j0, 32), 0), map, map + (int64_t)BH * QC * KC, MapLoad());
   __syncthreads();
   for (int t = r; t < kMask / 32; t += kListRows) {
     const int j = t * 32 + lane;

@@ -24,6 +24,31 @@ __device__ __forceinline__ float exp_f32_fixed(float x) {
   return __fmul_rn(p, __int_as_float((ni + 127) << 23));
 }
 
+// The `bytes` (at most 32) map bytes at `at` as aligned 32-bit words, first byte at byte `skew` (returned) of w[0]; the
+// other bytes of the words hold whatever lies there, or zeros.  [lo, hi) is the whole map: words that reach over its
+// start or end are put together from the bytes inside.  Load: how memory is read (the host test records it).
+struct MapLoad {
+  __host__ __device__ __forceinline__ uint32_t word(const uint8_t* p) const { return *reinterpret_cast<const uint32_t*>(p); }
+  __host__ __device__ __forceinline__ uint32_t byte(const uint8_t* p) const { return *p; }
+};
+template <class Load>
+__host__ __device__ __forceinline__ int map_words(uint32_t (&w)[9], const uint8_t* at, int bytes, const uint8_t* lo,
+                                                  const uint8_t* hi, const Load& load) {
+  const int skew = (int)(reinterpret_cast<uintptr_t>(at) & 3);
+  const int n = bytes > 0 ? (skew + bytes + 3) / 4 : 0;
+  const uint8_t* first = at - skew;
+  if (first >= lo && first + 4 * n <= hi) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) w[i] = i < n ? load.word(first + 4 * i) : 0;
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < 9; ++i) w[i] = 0;
+#pragma unroll 1
+    for (int b = skew; b < skew + bytes; ++b) w[b >> 2] |= load.byte(first + b) << (8 * (b & 3));
+  }
+  return skew;
+}
+
 struct HeadLimits {
   int32_t preserve[SVOO_MAX_HEADS];
   int32_t cap[SVOO_MAX_HEADS];

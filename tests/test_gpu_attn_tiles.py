@@ -116,3 +116,23 @@ def test_query_clusters_without_keys(rows):
     assert (got[dead] == 0).all()
     want = _reference(q[:1], k[:1], v[:1], sel[:1], qs[:1], ks[:1], 128 ** -0.5)
     assert (got[:1].float() - want).abs().max() <= 2.5 * 2.0 ** -9 * v.float().abs().max()
+
+
+@pytest.mark.parametrize("KC", [5, 33, 97, 1025])
+def test_map_at_any_address(KC):
+    """A map that starts and ends inside a 32-bit word gives the rows of an aligned one."""
+    from svoo_b200 import ops
+    dev = torch.device("cuda")
+    H, QC, S = 3, 3, 2053
+    gen = torch.Generator().manual_seed(KC)
+    qs, ks = (torch.full((H, c), S // c) for c in (QC, KC))
+    qs[:, 0] += S - qs[0].sum()
+    ks[:, 0] += S - ks[0].sum()
+    q, k, v = (torch.randn(H, S, 128, generator=gen).to(dev, torch.bfloat16) for _ in range(3))
+    m = (torch.rand(H, QC, KC, generator=gen) < 0.5).to(torch.uint8).to(dev)
+    want = ops.sparse_attn(q, k, v, m, _offsets(qs, dev), _offsets(ks, dev))
+    for shift in (1, 2, 3):
+        buf = torch.ones(m.numel() + 8, dtype=torch.uint8, device=dev)
+        view = buf[shift:shift + m.numel()].view(H, QC, KC)
+        view.copy_(m)
+        assert torch.equal(ops.sparse_attn(q, k, v, view, _offsets(qs, dev), _offsets(ks, dev)), want)
