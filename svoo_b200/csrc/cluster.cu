@@ -10,6 +10,8 @@
 // One GEMM [N,128] x [128,J] per side and iteration replaces the two chained GEMMs and
 // the separate norm pass.  W is carried as a bf16 pair (hi, lo = bf16(W - hi)) so the
 // products keep ~16 mantissa bits, more than the TF32 operands of the reference.
+#include <atomic>
+
 #include "common.cuh"
 
 namespace svoo {
@@ -222,8 +224,6 @@ __global__ void __launch_bounds__(256) profile_prologue_kernel(
 // ---------------------------------------------------------------------------------------
 constexpr int kSortWarps = 16;
 constexpr int kSortThreads = 32 * kSortWarps;
-constexpr int kSortCtasPerSm = 3;
-constexpr int kSortMaxCluster = 16;
 inline size_t sort_smem_bytes(int64_t K) { return (size_t)(kSortWarps + 2) * K * 4; }          // 72 KB at 1024 clusters
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
@@ -544,10 +544,39 @@ cudaError_t launch_prologue(const void* own, const void* form, void* w_hi, void*
                     (bf16*)w_lo, (int)J, (int)K, Jpad);
 }
 
+// Whether the device can place a cluster of `ctas` CTAs of the sort with the shared memory of the most clusters: sizes
+// above 8 are not portable, and a partition of a GPU has fewer SMs to a GPC.  Asked once per device, kernel form
+// and size; the answer is the device's.
+using SortKernel = void (*)(const int2*, int32_t*, int32_t*, int32_t*, int32_t*, int, int, int);
+static bool sort_cluster_fits(SortKernel kernel, int form, int dev, int ctas) {
+  constexpr int kDevices = 64;
+  static std::atomic<signed char> known[kDevices][5][5];                     // [log2 ctas]: 0 not asked, 1 yes, -1 no
+  std::atomic<signed char>* cell = dev < kDevices ? &known[dev][form][31 - __builtin_clz(ctas)] : nullptr;
+  const signed char before = cell ? cell->load(std::memory_order_relaxed) : 0;
+  if (before) return before > 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(kSortThreads);
+  cfg.dynamicSmemBytes = sort_smem_bytes(SVOO_MAX_CLUSTERS);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (cell) cell->store(n >= 1 ? 1 : -1, std::memory_order_relaxed);
+  return n >= 1;
+}
+
 // groups > 0: `labels` are first reduced from that many column groups of `partial` (see assign_tc.cu).
 cudaError_t launch_sort_labels(const int2* partial, int groups, int32_t* labels, int64_t BH, int64_t N, int64_t K,
                                int32_t* sorted_idx, int32_t* offsets, int32_t* sizes, cudaStream_t st) {
-  void (*kernel)(const int2*, int32_t*, int32_t*, int32_t*, int32_t*, int, int, int) = nullptr;
+  SortKernel kernel = nullptr;
   switch (groups) {                                      // two per 256 (at most 128 clusters: 128) W rows
     case 0: kernel = sort_labels_kernel<0>; break;
     case 2: kernel = sort_labels_kernel<2>; break;
@@ -563,12 +592,7 @@ cudaError_t launch_sort_labels(const int2* partial, int groups, int32_t* labels,
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // As many CTAs per head as surely fit the chip at once (a cluster stays inside one GPC, so the last quarter of
-  // the slots is not counted on), of at least 512 tokens and K (a CTA clears and scans 16 K counters).
-  // 24 heads x 8,505 tokens, 1024 clusters: 34 us with 16 CTAs per head, 16 us with 4.
-  const int64_t slots = (int64_t)sms * kSortCtasPerSm * 3 / 4, min_tokens = K > 512 ? K : 512;
-  int ctas = 1;
-  while (ctas < kSortMaxCluster && BH * ctas * 2 <= slots && N >= ctas * 2 * min_tokens) ctas *= 2;
+  const int ctas = sort_cluster_ctas(BH, N, K, sms, [&](int n) { return sort_cluster_fits(kernel, groups / 2, dev, n); });
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(BH * ctas));
   cfg.blockDim = dim3(kSortThreads);

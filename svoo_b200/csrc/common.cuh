@@ -52,6 +52,21 @@ __host__ inline bool single_tile_kernel_wins(int64_t S, int64_t QC) { return S <
 // 151, where TMA keeps up and the box count per tile is time lost: 2062 -> 2091 us at 5 x 75,600).
 __host__ inline bool short_key_runs(int64_t S, int64_t KC) { return S < 100 * KC; }
 
+// CTAs per head (one cluster) of the label sort: as many as surely fit the chip at once (a cluster stays inside one
+// GPC, so the last quarter of the slots is not counted on), of at least 512 tokens and K (a CTA clears and scans 16 K
+// counters), of a size that fits(ctas) says the device can place.
+// 24 heads x 8,505 tokens, 1024 clusters: 34 us with 16 CTAs per head, 16 us with 4.
+constexpr int kSortCtasPerSm = 3;
+constexpr int kSortMaxCluster = 16;
+template <class Fits>
+__host__ inline int sort_cluster_ctas(int64_t BH, int64_t N, int64_t K, int sms, Fits fits) {
+  const int64_t slots = (int64_t)sms * kSortCtasPerSm * 3 / 4, min_tokens = K > 512 ? K : 512;
+  int ctas = 1;
+  while (ctas < kSortMaxCluster && BH * ctas * 2 <= slots && N >= ctas * 2 * min_tokens) ctas *= 2;
+  while (ctas > 1 && !fits(ctas)) ctas /= 2;
+  return ctas;
+}
+
 __host__ inline Workspace workspace_layout(int64_t BH, int64_t N, int64_t QC, int64_t KC) {
   Workspace w;
   const int64_t Kmax = QC > KC ? QC : KC;

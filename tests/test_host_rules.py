@@ -47,6 +47,24 @@ int main() {
 """
 
 
+SORT_RULE = r"""
+#include <cstdio>
+#include "common.cuh"
+// The sort takes the largest cluster that the size asks for and the device can place.
+int main() {
+  const long sizes[][3] = {{1, 1, 1}, {2, 4096, 32}, {12, 32760, 500}, {40, 75600, 500}, {3, 40003, 1024}, {300, 75600, 100}};
+  const int want[] = {1, 8, 16, 8, 16, 1};
+  for (int i = 0; i < 6; ++i)
+    for (int limit = 1; limit <= 16; limit *= 2) {
+      const int got = svoo::sort_cluster_ctas(sizes[i][0], sizes[i][1], sizes[i][2], 148, [&](int ctas) { return ctas <= limit; });
+      if (got != (want[i] < limit ? want[i] : limit)) return printf("%d %d: %d\n", i, limit, got), 1;
+    }
+  puts("ok");
+  return 0;
+}
+"""
+
+
 def _run(tmp_path, source):
     src, exe = tmp_path / "t.cu", tmp_path / "t"
     src.write_text(source)
@@ -59,3 +77,7 @@ def _run(tmp_path, source):
 
 def test_map_words_stay_inside_the_map(tmp_path):
     _run(tmp_path, MAP_READS)
+
+
+def test_sort_takes_a_cluster_that_fits(tmp_path):
+    _run(tmp_path, SORT_RULE)
