@@ -162,6 +162,10 @@ class _SAPBase:
     def flash_attention(self, query, key, value):
         return F.scaled_dot_product_attention(query, key, value, dropout_p=0.0, is_causal=False)
 
+    # whether attention_core_logic returns [1, S, H*128]: the attention then stores its rows token-major, which makes
+    # the transpose behind it a view
+    _token_major = False
+
     def _sparse(self, query, key, value, prompt_length=None):
         cfg, H, S, D = query.shape
         n_video = self.num_frame * self.frame_size
@@ -170,9 +174,8 @@ class _SAPBase:
         extra = 2 if self.context_length else 0
         self._last_shape = (query.device, cfg * H, S, n_video, self.num_q_centroids + extra, self.num_k_centroids + extra)
         ratio = self._get_min_kc_ratio_for_heads_from_step(self.current_inference_step, H)
-        # the attention stores its rows token-major, so that the callers' transpose(1, 2).flatten(2, 3) is a view
         rows, peer_out = None, None
-        if cfg == 1 and H <= 128:
+        if self._token_major and cfg == 1 and H <= 128:
             rows = torch.empty(cfg, S, H, D, dtype=query.dtype, device=query.device)
             peer_out = ops.token_major(rows)
         out, state = sparse_attention_layer(query, key, value, num_q_centroids=self.num_q_centroids,
@@ -189,6 +192,7 @@ class _SAPBase:
 
 class WanAttn_SAPAttn_Processor(_SAPBase):
     """Self-attention processor for Wan DiT blocks; cross attention (timestep is None) is dense."""
+    _token_major = True
 
     def get_qkv(self, attn, hidden_states, encoder_hidden_states):
         if encoder_hidden_states is None:

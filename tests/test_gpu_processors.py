@@ -418,3 +418,26 @@ def test_hunyuan_fused_producer_equals_module_path(dev, double_stream):
         assert (x - r).abs().max() <= 2.0 ** -5 * max(1.0, float(r.abs().max()))
     assert torch.equal(a[0]["v"], b[0]["v"])
     assert (a[1].float() - b[1].float()).abs().max() <= 3e-2 and (a[2].float() - b[2].float()).abs().max() <= 3e-2
+
+
+@pytest.mark.parametrize("timestep", [10.0, 2e9])
+@pytest.mark.parametrize("name", ["Hunyuan_SAPAttn_Processor2_0", "WanAttn_SAPAttn_Processor"])
+def test_core_logic_results_are_contiguous(dev, name, timestep):
+    """attention_core_logic returns a tensor that a caller may view(), in the sparse and in the dense branch."""
+    from svoo_b200 import processor
+    cls = _fresh(getattr(processor, name))
+    joint = name.startswith("Hunyuan")
+    text = 64 if joint else 0
+    cfg = dataclasses.replace(gu.TINY_BF16, text_tokens=text, cfg_id=95)
+    cls.num_frame, cls.frame_size, cls.context_length = cfg.grid[0], cfg.grid[1] * cfg.grid[2], text
+    cls.num_q_centroids, cls.num_k_centroids, cls.top_p_kmeans, cls.min_kc_ratio = cfg.num_q, cfg.num_k, 0.9, 0.2
+    cls.kmeans_iter_init = cls.kmeans_iter_step = 2
+    cls.first_times_fp = 1e9
+    if joint:
+        cls.prompt_length = 40
+    q, k, v = (t.to(dev) for t in synth.make_qkv(cfg))
+    H, S = q.shape[1:3]
+    out = cls(0).attention_core_logic(q, k, v, torch.tensor([timestep], device=dev))
+    assert out.shape == ((1, H, S, 128) if joint else (1, S, H * 128))
+    assert out.is_contiguous() and out.dtype == q.dtype
+    out.view(-1, 128)
