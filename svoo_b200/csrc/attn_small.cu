@@ -3,8 +3,8 @@
 //
 // attn_tc.cu owns pairs of query tiles: one CTA per SM, two softmax warpgroups that hide each other's
 // latency, K and V by TMA boxes.  A single tile in that kernel leaves half of the CTA idle and pays for
-// every wait.  Here a CTA owns one query tile and walks 64-key steps with 97 KB of shared memory and
-// 256 TMEM columns, so that TWO CTAs share an SM and cover each other's waits, start and end.
+// every wait.  Here a CTA owns one query tile and walks 64-key steps with 102 KB of shared memory (106 KB
+// in the EAR form) and 256 TMEM columns, so that TWO CTAs share an SM and cover each other's waits, start and end.
 //
 //   warps 0-3   softmax: thread r owns row r; S -> registers, row max, exp2, row sum, P packed to bf16
 //               over the S columns it came from
@@ -15,6 +15,11 @@
 // rows is a handful of rows long and a 128-key tile takes about 35 TMA boxes per tensor, which at 113
 // cycles a box is the whole time (hunyuan-shaped layer, 24 heads x 8,505 tokens: 4.5 us per tile against
 // 1.9 us when the same number of selected rows is contiguous).  A gather costs the same for any run.
+//
+// The softmax takes its maximum over 128 keys (two steps), as the pair kernel does, and adds in the same order, so that
+// a row comes out the same bit for bit in either kernel.  A maximum per 64-key step would be simpler, but the key that is
+// the maximum has P = 1, which bf16 holds exactly, and is found in the first step less often: 0.5 % more error
+// against 64 bits at 4 heads x 960 tokens.
 #include "attn_common.cuh"
 
 namespace svoo {
@@ -38,8 +43,8 @@ struct SmallSmem {
 };
 static_assert(2 * (SmallSmem<true>::kBytes + 1024) <= 228 * 1024, "two CTAs share an SM");
 
-// PV_DONE has one barrier per step parity because the softmax does not wait for every PV: when it asks
-// for step j, step j - 2 is known to be complete (S of step j was issued after it) but step j - 1 is not.
+// PV_DONE has one barrier per step parity because the softmax does not wait for every PV: when it has S of
+// step j, the PV of step j - 2 is known to be complete (S of step j was issued after it).
 enum SmBar { SM_Q_FULL = 0, SM_K_FULL = 1, SM_K_EMPTY = 3, SM_V_FULL = 5, SM_V_EMPTY = 7, SM_S_FULL = 9, SM_P_READY = 11,
              SM_PV_DONE = 13, SM_NUM_BARS = 15 };
 // TMEM columns: two S buffers (P of a step overwrites the first half of its S buffer), then O.
@@ -211,40 +216,76 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
     float m_used = -INFINITY, l_sum = 0.f;
     bool ok = true;
     const uint64_t scale2 = pair2(scale_log2);
-    for (int j = 0; j < T; ++j) {
-      const uint32_t s_t = tmem + lane_addr + (j & 1) * kSmBN;   // S, then P of this step
-      const int valid = min(L - j * kSmBN, kSmBN);
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(SM_S_FULL + (j & 1)), (j >> 1) & 1, abort_flag));
+    const int bias_step = l_tok / kSmBN;                          // first step with centroid keys (EAR)
+    // f(c, scores [16 c, 16 c + 16) of step j) for the four quarters of a step in order, bias and end of the list applied;
+    // a quarter is read while the one before it is worked on.
+    auto quarters = [&](int j, auto f) {
+      const uint32_t s_t = tmem + lane_addr + (j & 1) * kSmBN;
+      const bool biased = kEar && j >= bias_step;
+      uint32_t sc[2][16];
+      tmem_ld16_nowait(s_t, sc[0]);
+      tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t(&x)[16] = sc[c & 1];
+        if (c < 3) tmem_ld16_nowait(s_t + 16 * (c + 1), sc[(c + 1) & 1]);
+        if (biased) {
+          const uint32_t bj = base + kSmTiles + 256 + SmallSmem<kEar>::kRunTableBytes + 4u * ((j - bias_step) * kSmBN + c * 16);
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            float b0, b1;
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(b0), "=f"(b1) : "r"(bj + 4 * i));
+            x[i] = __float_as_uint(__uint_as_float(x[i]) + b0);
+            x[i + 1] = __float_as_uint(__uint_as_float(x[i + 1]) + b1);
+          }
+        }
+        const int valid = L - j * kSmBN - c * 16;
+        if (valid < 16) {                                         // last step only: columns past the last key
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (i >= valid) x[i] = 0xff800000u;
+        }
+        f(c, x);
+        tmem_wait_ld();
+      }
+    };
+    auto max16 = [](const uint32_t (&x)[16], float& m0, float& m1) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        m0 = fmaxf(m0, fmaxf(__uint_as_float(x[i]), __uint_as_float(x[i + 1])));
+        m1 = fmaxf(m1, fmaxf(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])));
+      }
+    };
+    // 128 keys: both steps' maxima decide on the maximum before any of their P goes to the tensor core.  It rarely
+    // changes after the first 128 keys, so the first step's P is computed on the old one while the second step's S is
+    // still being formed, kept in registers, and computed again if the maximum did change.
+    for (int j0 = 0; j0 < T; j0 += 2) {
+      const uint32_t par = (j0 >> 1) & 1;
+      uint32_t pk[32];
+      uint64_t acc = 0;                                           // two fp32 zeros
+      float m0 = -INFINITY, m1 = -INFINITY;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(SM_S_FULL), par, abort_flag));
       if (!ok) break;
       tc_fence_after();
-      uint32_t sc[64];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) tmem_ld32_nowait(s_t + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&sc[c * 32]));
-      tmem_wait_ld();
-      if (kEar && (j + 1) * kSmBN > l_tok) {                      // a step with centroid keys
-        const float* bj = bias_s + (j * kSmBN - bias0);
-#pragma unroll
-        for (int i = 0; i < 64; ++i) sc[i] = __float_as_uint(__uint_as_float(sc[i]) + bj[i]);
+      bool have_p = j0 > 0;
+      quarters(j0, [&](int c, const uint32_t (&x)[16]) {
+        max16(x, m0, m1);
+        if (have_p) have_p = !__any_sync(0xffffffffu, lane_has_row && fmaxf(m0, m1) * scale_log2 > m_used + kRescaleThreshold);
+        if (have_p) exp_pack16(x, &pk[c * 8], scale2, pair2(-m_used), acc);
+      });
+      if (j0 + 1 < T) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(SM_S_FULL + 1), par, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        quarters(j0 + 1, [&](int, const uint32_t (&x)[16]) { max16(x, m0, m1); });
       }
-      if (valid < kSmBN) {                                        // last step only: columns past the last key
-#pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (i >= valid) sc[i] = 0xff800000u;
-      }
-      float mr[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int i = 0; i < 64; i += 8) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          mr[u] = fmaxf(mr[u], fmaxf(__uint_as_float(sc[i + 2 * u]), __uint_as_float(sc[i + 2 * u + 1])));
-      }
-      const float m_tile = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * scale_log2;   // the scale is positive
-      if (j == 0) {
-        m_used = kEar ? fmaxf(m_tile, -1e30f) : m_tile;           // EAR: a first step of masked centroids only
+      const float m_tile = fmaxf(m0, m1) * scale_log2;            // the scale is positive
+      if (j0 == 0) {
+        m_used = kEar ? fmaxf(m_tile, -1e30f) : m_tile;           // EAR: first steps of masked centroids only
       } else {
         const bool need = lane_has_row && m_tile > m_used + kRescaleThreshold;
         if (__any_sync(0xffffffffu, need)) {                      // rare: rescale O once the previous PV is complete
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(SM_PV_DONE + ((j - 1) & 1)), ((j - 1) >> 1) & 1, abort_flag));
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(SM_PV_DONE + 1), par ^ 1, abort_flag));
           if (!ok) break;
           tc_fence_after();
           const float alpha = need ? fast_exp2(m_used - m_tile) : 1.0f;
@@ -258,22 +299,28 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
           }
           l_sum *= alpha;
           if (need) m_used = m_tile;
+          have_p = false;
         }
       }
       const uint64_t negm2 = pair2(-m_used);
-      uint64_t acc = 0;                                           // two fp32 zeros
-#pragma unroll
-      for (int c = 0; c < 4; c += 2) {
-        uint32_t pk[16];
-        exp_pack16(*reinterpret_cast<const uint32_t(*)[16]>(&sc[c * 16]), &pk[0], scale2, negm2, acc);
-        exp_pack16(*reinterpret_cast<const uint32_t(*)[16]>(&sc[(c + 1) * 16]), &pk[8], scale2, negm2, acc);
-        tmem_st16(s_t + c * 8, pk);
+      auto hand_over = [&](int u) {                               // P over the S it came from
+        tmem_st16(tmem + lane_addr + u * kSmBN, *reinterpret_cast<const uint32_t(*)[16]>(&pk[0]));
+        tmem_st16(tmem + lane_addr + u * kSmBN + 16, *reinterpret_cast<const uint32_t(*)[16]>(&pk[16]));
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(SM_P_READY + u));
+      };
+      if (have_p)
+        hand_over(0);
+      else
+        acc = 0;
+#pragma unroll 1
+      for (int u = have_p ? 1 : 0; u < min(T - j0, 2); ++u) {
+        quarters(j0 + u, [&](int c, const uint32_t (&x)[16]) { exp_pack16(x, &pk[c * 8], scale2, negm2, acc); });
+        hand_over(u);
       }
       l_sum += pair_sum(acc);
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(SM_P_READY + (j & 1)));
     }
     // epilogue: O / l -> bf16 rows
     const int row = row0 + r_local;
@@ -326,7 +373,9 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
 
 }  // namespace tc
 
-// after_pairs: the pair kernel of the same call was launched just before on this stream.
+// after_pairs: the pair kernel of the same call was launched just before on this stream, as an ordinary launch behind
+// the lists.  This one then starts beside it and needs no wait for the lists: they were complete before the pair
+// kernel began, and it begins after that.  Only the last CTA waits, for the pair kernel's end.
 cudaError_t launch_sparse_attn_small(const CUtensorMap& q_map, const tc::OutPeers& peers, const void* k, const void* v,
                                      void* out, const int32_t* out_row_idx, const int4* qtiles, const int32_t* nqtiles,
                                      const int32_t* head_order, const int2* runs, const int32_t* nruns, int32_t* status, int64_t BH, int64_t S,

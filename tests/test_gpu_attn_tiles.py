@@ -136,3 +136,36 @@ def test_map_at_any_address(KC):
         view = buf[shift:shift + m.numel()].view(H, QC, KC)
         view.copy_(m)
         assert torch.equal(ops.sparse_attn(q, k, v, view, _offsets(qs, dev), _offsets(ks, dev)), want)
+
+
+@pytest.mark.parametrize("keys", ["short", "long", "rising"])
+@pytest.mark.parametrize("ear", [False, True])
+def test_single_tiles_are_the_same_in_either_kernel(keys, ear):
+    """Two empty query clusters more and the single tiles go to their own kernel instead of the pair kernel: the same
+    bits, output and log-sum-exp.  `rising`: row maxima that grow along the keys, so that O is rescaled, first in one
+    half of a 128-key tile and then in the other."""
+    from svoo_b200 import ops
+    dev = torch.device("cuda")
+    qsz = [100, 28, 64, 65, 1, 3712]                              # the last one leaves a remainder of 128 rows
+    ksz = [3, 40, 1, 96, 5, 7] * 26 + [18] if keys == "short" else [400, 1, 63, 64, 2, 130, 900, 2410]
+    H, S, QC, KC = 2, 3970, len(qsz), len(ksz)
+    assert sum(qsz) == sum(ksz) == S and 640 * QC <= S < 640 * (QC + 2)
+    gen = torch.Generator().manual_seed(KC)
+    q, k, v = (torch.randn(H, S, 128, generator=gen) for _ in range(3))
+    if keys == "rising":
+        k = k * torch.linspace(0.2, 6.0, S)[None, :, None]
+    q, k, v = (t.to(dev, torch.bfloat16) for t in (q, k, v))
+    kc, vc = (torch.randn(H * KC, 128, generator=gen).to(dev, torch.bfloat16) for _ in range(2))
+    sel = (torch.rand(H, QC + 2, KC, generator=gen) < 0.6).to(torch.uint8)
+    sel[..., 0] = 1
+    k_off = _offsets(torch.tensor([ksz] * H), dev)
+    got = []
+    for extra in (0, 2):
+        q_off = _offsets(torch.tensor([qsz + [0] * extra] * H), dev)
+        m = sel[:, :QC + extra].contiguous().to(dev)
+        if ear:
+            got.append(ops.sparse_attn_ear(q, torch.cat([k.view(-1, 128), kc]), torch.cat([v.view(-1, 128), vc]), m, q_off,
+                                           k_off, return_lse=True))
+        else:
+            got.append(ops.sparse_attn(q, k, v, m, q_off, k_off, return_lse=True))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
