@@ -555,7 +555,7 @@ cudaError_t launch_sparse_attn_tc(const void* q, const void* k, const void* v, v
   const float scale_log2 = sm_scale * 1.4426950408889634f;
   const int runs_per_row = ear ? ear_max_runs : max_runs(KC);
   if (peer_dst) lse = nullptr;
-  const bool split = single_tile_kernel_wins(S, QC);
+  const bool split = single_tile_kernel_wins(S, QC, ear);
   // tiles per head: of at least 129 rows each, or a cluster's whole 256-row tiles and its remainder
   const int per_head = (int)(split ? S / (tc::kBM + 1) : S / (2 * tc::kBM) + QC);
   if (per_head > 0) {
@@ -566,6 +566,7 @@ cudaError_t launch_sparse_attn_tc(const void* q, const void* k, const void* v, v
     const int smem = ear ? tc::AttnSmem<true>::kBytes : tc::AttnSmem<false>::kBytes;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
+    // not launch_pdl(): the single-tile kernel behind it relies on the lists being complete when this one begins
     kernel<<<(unsigned)(BH * per_head), tc::kThreads, smem, st>>>(
         maps, peers, (const bf16*)k, (const bf16*)v, (bf16*)out, out_row_idx, qtiles, nqtiles, head_order, runs, nruns, (int)BH, (int)S,
         (int)QC, max_qtiles(S, QC), per_head, runs_per_row, scale_log2, status, lse, ear_map, ear_k_offsets, (int)KC,

@@ -43,14 +43,18 @@ __host__ inline int pad_clusters(int64_t K) { return (int)align_up(K, 256); }   
 __host__ inline int max_runs(int64_t KC) { return (int)(KC / 2 + 2); }   // + one sentinel entry
 __host__ inline int max_qtiles(int64_t N, int64_t QC) { return (int)(ceil_div64(N, kAttnBM) + QC); }
 
-// Query tiles of at most 128 rows go to the kernel of attn_small.cu, unless they are the few remainders of
-// large query clusters.  Attention of 10 x 20,000 tokens with 256 / 160 clusters (78 rows per query cluster):
-// 914 -> 632 us; 12 x 32,760, 100 / 500 (328 rows): 1630 -> 1483; 8 x 59,400, 100 / 800 (594): 2752 -> 2717;
-// 5 x 75,600, 100 / 500 (756): 2129 -> 2157.
-__host__ inline bool single_tile_kernel_wins(int64_t S, int64_t QC) { return S < 640 * QC; }
-// Mean key cluster of at most 100 rows: tiles of too many TMA boxes occur (14 boxes per tile at 65 rows, 9 at
-// 151, where TMA keeps up and the box count per tile is time lost: 2062 -> 2091 us at 5 x 75,600).
-__host__ inline bool short_key_runs(int64_t S, int64_t KC) { return S < 100 * KC; }
+// Query tiles of at most 128 rows go to the kernel of attn_small.cu where query clusters are small on average.  Time with
+// the split over time without, clustered video tokens, budgets 0.1 to 0.2, key clusters of 32 / 65 / 120 rows:
+//   60 rows per query cluster   12 x 32,760 tokens 0.64 / 0.86 / 0.90   12 x 12,150 0.53 / 0.78 / 0.83   2 x 32,760 0.64 / 0.83 / 0.87
+//   130                                     0.85 / 1.01 / 1.06                      0.83 / 0.94 / 1.00              0.84 / 0.98 / 0.99
+//   200                                     0.94 / 1.02 / 1.01                      0.99 / 1.03 / 1.04              1.10 / 1.20 / 1.23
+// With error-aware routing (every list ends with one long run of centroid keys) the two meet earlier: at 130 rows 0.96 / 1.02 / 1.04,
+// 0.90 / 1.00 / 1.04, 0.89 / 1.03 / 1.02.
+__host__ inline bool single_tile_kernel_wins(int64_t S, int64_t QC, bool ear) { return S < (ear ? 100 : 150) * QC; }
+// The pair kernel gathers key tiles of many short runs with cp.async below 42 rows per key cluster.  With over without,
+// same tokens: 0.85 to 0.97 at 32 rows, 1.01 to 1.06 at 45 (finding out costs more than the boxes that are saved); a whole
+// Wan block of 12 x 20,280 tokens at 41 rows 2010 -> 1993 us.
+__host__ inline bool short_key_runs(int64_t S, int64_t KC) { return S < 42 * KC; }
 
 // CTAs per head (one cluster) of the label sort: as many as surely fit the chip at once (a cluster stays inside one
 // GPC, so the last quarter of the slots is not counted on), of at least 512 tokens and K (a CTA clears and scans 16 K

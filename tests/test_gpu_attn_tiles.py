@@ -138,29 +138,33 @@ def test_map_at_any_address(KC):
         assert torch.equal(ops.sparse_attn(q, k, v, view, _offsets(qs, dev), _offsets(ks, dev)), want)
 
 
-@pytest.mark.parametrize("keys", ["short", "long", "rising"])
+@pytest.mark.parametrize("name", ["short", "long", "rising"] + list(CASES))
 @pytest.mark.parametrize("ear", [False, True])
-def test_single_tiles_are_the_same_in_either_kernel(keys, ear):
-    """Two empty query clusters more and the single tiles go to their own kernel instead of the pair kernel: the same
+def test_single_tiles_are_the_same_in_either_kernel(name, ear):
+    """Empty query clusters more and the single tiles go to their own kernel instead of the pair kernel: the same
     bits, output and log-sum-exp.  `rising`: row maxima that grow along the keys, so that O is rescaled, first in one
     half of a 128-key tile and then in the other."""
     from svoo_b200 import ops
     dev = torch.device("cuda")
-    qsz = [100, 28, 64, 65, 1, 3712]                              # the last one leaves a remainder of 128 rows
-    ksz = [3, 40, 1, 96, 5, 7] * 26 + [18] if keys == "short" else [400, 1, 63, 64, 2, 130, 900, 2410]
-    H, S, QC, KC = 2, 3970, len(qsz), len(ksz)
-    assert sum(qsz) == sum(ksz) == S and 640 * QC <= S < 640 * (QC + 2)
+    if name in CASES:
+        qsz, ksz, _ = CASES[name]
+    else:
+        qsz = [100, 28, 64, 65, 1, 3712]                          # the last one leaves a remainder of 128 rows
+        ksz = [3, 40, 1, 96, 5, 7] * 26 + [18] if name == "short" else [400, 1, 63, 64, 2, 130, 900, 2410]
+    H, S, QC, KC = 2, sum(qsz), len(qsz), len(ksz)
+    more = 40                                                     # split below 100 (error-aware) / 150 rows per query cluster
+    assert sum(ksz) == S < 100 * (QC + more) and (name in CASES or S >= 150 * QC)
     gen = torch.Generator().manual_seed(KC)
     q, k, v = (torch.randn(H, S, 128, generator=gen) for _ in range(3))
-    if keys == "rising":
+    if name == "rising":
         k = k * torch.linspace(0.2, 6.0, S)[None, :, None]
     q, k, v = (t.to(dev, torch.bfloat16) for t in (q, k, v))
     kc, vc = (torch.randn(H * KC, 128, generator=gen).to(dev, torch.bfloat16) for _ in range(2))
-    sel = (torch.rand(H, QC + 2, KC, generator=gen) < 0.6).to(torch.uint8)
+    sel = (torch.rand(H, QC + more, KC, generator=gen) < 0.6).to(torch.uint8)
     sel[..., 0] = 1
     k_off = _offsets(torch.tensor([ksz] * H), dev)
     got = []
-    for extra in (0, 2):
+    for extra in (0, more):
         q_off = _offsets(torch.tensor([qsz + [0] * extra] * H), dev)
         m = sel[:, :QC + extra].contiguous().to(dev)
         if ear:
