@@ -218,12 +218,19 @@ __global__ void __launch_bounds__(256) profile_prologue_kernel(
 // (lower group wins ties) and written out on the way.
 //
 // As separate histogram, scan and scatter kernels this was three of the seven launches of a clustering
-// phase, each of them a chain of dependent loads.  Mean of both sides, 100 / 500 clusters: 12 x 32,760 tokens
-// 19.2 -> 11.3 us, 5 x 75,600 20.6 -> 15.2, 40 x 75,600 55 -> 47; 2 x 4,096, 32 / 128: 12.4 -> 6.4.  What is left
-// is shared-memory work: an atomic per token in the first walk, a match and two accesses in the second.
+// phase, each of them a chain of dependent loads.  Labels alone, before -> now: 12 x 32,760 tokens, 100 / 1024 clusters
+// 14.2 -> 9.7 / 16.9 -> 13.3 us, 40 x 75,600, 100 / 500 clusters 34.9 -> 28.2 / 43.2 -> 32.6, 24 x 118,800, 500 clusters
+// 44.9 -> 35.7, 1 x 4,096 tokens, 100 clusters 9.5 -> 5.5.  What is left is shared-memory work (an atomic per token in the first walk, two
+// accesses in the second) and the scattered stores.  One head has 16 CTAs at most: with one million tokens a head and fewer
+// than five heads the three kernels were faster (1 x 1,000,000, 100 clusters: 39 against 67 us).
 // ---------------------------------------------------------------------------------------
 constexpr int kSortWarps = 16;
 constexpr int kSortThreads = 32 * kSortWarps;
+// Up to this many labels every CTA of the cluster reads the totals of all (one barrier less on the way); above, that is most
+// of the time once an SM holds several CTAs (16 CTAs: 64 KB of remote reads each at 1024 labels) and each does a share
+// for all.  Direct / shared: 12 x 75,600 tokens, 100 labels 18.2 / 19.1 us, 500 labels 22.7 / 21.2, 1024 labels 32.9 / 22.9.
+constexpr int kSortDirect = 256;
+static_assert(kSortDirect <= kSortThreads, "one label per thread");
 inline size_t sort_smem_bytes(int64_t K) { return (size_t)(kSortWarps + 2) * K * 4; }          // 72 KB at 1024 clusters
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
@@ -237,14 +244,34 @@ __device__ __forceinline__ int ld_cluster(uint32_t addr, uint32_t rank) {
   return v;
 }
 
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, int v) {
+  asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.s32 [a], %2;\n\t}\n"
+               ::"r"(addr), "r"(rank), "r"(v) : "memory");
+}
+
+// Lanes whose label equals this lane's; `bits` = width of a label.  A vote per bit: __match_any_sync takes time for every
+// different value among the lanes, and with it the second walk was most of the kernel.
+__device__ __forceinline__ unsigned same_label(int label, bool ok, int bits) {
+  unsigned grp = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+  for (int b = 0; b < 10; ++b) {                         // labels are below SVOO_MAX_CLUSTERS = 2^10
+    if (b < bits) {
+      const bool one = (label >> b) & 1;
+      const unsigned v = __ballot_sync(0xffffffffu, one);
+      grp &= one ? v : ~v;
+    }
+  }
+  return grp;
+}
+
 template <int kGroups>
 __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kernel(
     const int2* __restrict__ partial, int32_t* labels, int32_t* __restrict__ sorted_idx, int32_t* __restrict__ offsets,
     int32_t* __restrict__ sizes, int BH, int N, int K) {
   extern __shared__ int sort_sm[];
   int* wh = sort_sm;                                     // [16][K] counts, then positions, per warp
-  int* tot = wh + kSortWarps * K;                        // [K] this CTA's totals
-  int* add = tot + K;                                    // [K] first position of this CTA's tokens of a label
+  int* tot = wh + kSortWarps * K;                        // [K] this CTA's totals, then the head's
+  int* add = tot + K;                                    // [K] tokens of the CTAs before this one, then first positions
   __shared__ int warp_tot[kSortWarps];
   pdl_trigger();
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
@@ -310,30 +337,56 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
   cluster_arrive();
   cluster_wait();
 
-  // ---- totals of the head and of the CTAs before this one; exclusive scan over the labels
+  // ---- tokens of the head and of the CTAs before this one, per label
   constexpr int kPer = (SVOO_MAX_CLUSTERS + kSortThreads - 1) / kSortThreads;
   const int per = ceil_div(K, kSortThreads);             // labels per thread
-  int all[kPer], before[kPer], sum = 0;
-#pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int k = tid * per + u;
-    all[u] = before[u] = 0;
-    if (u < per && k < K)
+  int all[kPer] = {}, before[kPer] = {}, sum = 0;
+  if (K <= kSortDirect) {                                // every CTA reads everybody's totals
+    if (tid < K)
       for (int r0 = 0; r0 < ctas; r0 += 8) {             // eight remote reads in flight
         int v[8];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = ld_cluster(smem_u32(tot + k), min(r0 + r, ctas - 1));
+        for (int r = 0; r < 8; ++r) v[r] = r0 + r < ctas ? ld_cluster(smem_u32(tot + tid), r0 + r) : 0;
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-          if (r0 + r >= ctas) v[r] = 0;
-          if (r0 + r < rank) before[u] += v[r];
-          all[u] += v[r];
+          if (r0 + r < rank) before[0] += v[r];
+          all[0] += v[r];
         }
       }
-    sum += all[u];
+    __syncwarp();
+    cluster_arrive();                                    // this CTA has read the others' totals (waited for at the end)
+  } else {                                               // every CTA does its share of the labels for all of them
+    const int share = ceil_div(K, ctas), k1 = min((rank + 1) * share, K);
+    for (int k = rank * share + tid; k < k1; k += kSortThreads) {
+      int run = 0;
+      for (int r0 = 0; r0 < ctas; r0 += 8) {
+        int v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[r] = r0 + r < ctas ? ld_cluster(smem_u32(tot + k), r0 + r) : 0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if (r0 + r < ctas) st_cluster(smem_u32(add + k), r0 + r, run);
+          run += v[r];
+        }
+      }
+      for (int r = 0; r < ctas; ++r) st_cluster(smem_u32(tot + k), r, run);
+    }
+    __syncwarp();
+    cluster_arrive();                                    // nothing remote after this barrier
+    cluster_wait();
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int k = tid * per + u;
+      if (u < per && k < K) {
+        all[u] = tot[k];
+        before[u] = add[k];
+      }
+    }
   }
-  __syncwarp();
-  cluster_arrive();                                      // this CTA has read the others' totals (waited for at the end)
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) sum += all[u];
+
+  // ---- exclusive scan over the labels
   int incl = sum;
 #pragma unroll
   for (int s = 1; s < 32; s <<= 1) {
@@ -365,6 +418,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
 
   // ---- walk 2: the warp's tokens to their places, in order
   int32_t* out = sorted_idx + (int64_t)bh * N;
+  const int bits = 32 - __clz(K - 1);
   for (int s = w0; s < w1; s += 32 * 4) {
     int l[4];
 #pragma unroll
@@ -375,7 +429,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const bool ok = l[u] >= 0 && l[u] < K;
-      const unsigned grp = __match_any_sync(0xffffffffu, ok ? l[u] : K + lane);
+      const unsigned grp = same_label(l[u], ok, bits);
       const int pos_in_grp = __popc(grp & ((1u << lane) - 1u));
       int base = 0;
       if (ok) base = mine[l[u]];
@@ -388,8 +442,10 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
       }
     }
   }
-  __syncwarp();
-  cluster_wait();
+  if (K <= kSortDirect) {
+    __syncwarp();
+    cluster_wait();
+  }
 }
 
 // ---------------------------------------------------------------------------------------

@@ -58,15 +58,18 @@ __host__ inline bool short_key_runs(int64_t S, int64_t KC) { return S < 42 * KC;
 
 // CTAs per head (one cluster) of the label sort: as many as surely fit the chip at once (a cluster stays inside one
 // GPC, so the last quarter of the slots is not counted on), of at least 512 tokens and K (a CTA clears and scans 16 K
-// counters), of a size that fits(ctas) says the device can place.
-// 24 heads x 8,505 tokens, 1024 clusters: 34 us with 16 CTAs per head, 16 us with 4.
+// counters), of a size that fits(ctas) says the device can place.  Where a CTA still has 6,144 tokens, up to four CTAs per SM
+// in all, some of which then wait for a slot: 64 heads x 75,600 tokens, 100 clusters 53 -> 42 us, 24 x 118,800 34 -> 31.5;
+// with fewer tokens that loses (40 x 75,600, 45 -> 54; 24 x 8,505, 40 clusters, 8.8 with 8 CTAs per head, 13.3 with 16).
 constexpr int kSortCtasPerSm = 3;
 constexpr int kSortMaxCluster = 16;
 template <class Fits>
 __host__ inline int sort_cluster_ctas(int64_t BH, int64_t N, int64_t K, int sms, Fits fits) {
   const int64_t slots = (int64_t)sms * kSortCtasPerSm * 3 / 4, min_tokens = K > 512 ? K : 512;
   int ctas = 1;
-  while (ctas < kSortMaxCluster && BH * ctas * 2 <= slots && N >= ctas * 2 * min_tokens) ctas *= 2;
+  while (ctas < kSortMaxCluster && N >= ctas * 2 * min_tokens &&
+         (BH * ctas * 2 <= slots || (N >= ctas * 2 * 6144 && BH * ctas * 2 <= 4 * (int64_t)sms)))
+    ctas *= 2;
   while (ctas > 1 && !fits(ctas)) ctas /= 2;
   return ctas;
 }
@@ -98,12 +101,14 @@ inline void count_launches(int n) { __atomic_fetch_add(&launch_counter(), (int64
 
 // ---------------------------------------------------------------------------------------
 // Programmatic dependent launch.  The clustering is a chain of short kernels (ten phases of
-// seven launches); launched this way, a kernel's CTAs are scheduled and run their set-up while
+// five launches); launched this way, a kernel's CTAs are scheduled and run their set-up while
 // the previous kernel drains, and block in pdl_wait() until that kernel has completed and its
 // writes are visible.  Every kernel launched with launch_pdl() calls pdl_wait() before its first
 // access to memory that an earlier kernel of the stream wrote, and pdl_trigger() at its start
 // (the next kernel's CTAs may then be scheduled as soon as every CTA of this one has started).
 // Outside such a launch both are no-ops.
+// One exception: sparse_attn_small_kernel reads the lists of attn_lists_kernel without waiting.  The pair kernel
+// between the two must therefore be an ordinary launch, which starts when the lists are complete (see both launch sites).
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -38,7 +38,7 @@ def test_sort_reduces_the_assignment_winners(J):
     assert torch.equal(c.ksizes.long(), torch.stack([torch.bincount(r, minlength=J) for r in klab.long()]))
 
 
-@pytest.mark.parametrize("K", [1, 31, 33, 500, 511, 513, 1023])
+@pytest.mark.parametrize("K", [1, 31, 33, 256, 257, 500, 511, 513, 1023])
 def test_sort_of_sixteen_ctas_with_partial_warps(K):
     """Sixteen CTAs per head with cluster counts that end inside a warp: its lanes meet the cluster barriers from
     loops of different lengths."""

@@ -52,9 +52,9 @@ SORT_RULE = r"""
 #include "common.cuh"
 // The sort takes the largest cluster that the size asks for and the device can place.
 int main() {
-  const long sizes[][3] = {{1, 1, 1}, {2, 4096, 32}, {12, 32760, 500}, {40, 75600, 500}, {3, 40003, 1024}, {300, 75600, 100}};
-  const int want[] = {1, 8, 16, 8, 16, 1};
-  for (int i = 0; i < 6; ++i)
+  const long sizes[][3] = {{1, 1, 1}, {2, 4096, 32}, {12, 32760, 500}, {40, 75600, 500}, {3, 40003, 1024}, {64, 75600, 100}, {300, 75600, 100}};
+  const int want[] = {1, 8, 16, 8, 16, 8, 1};
+  for (int i = 0; i < 7; ++i)
     for (int limit = 1; limit <= 16; limit *= 2) {
       const int got = svoo::sort_cluster_ctas(sizes[i][0], sizes[i][1], sizes[i][2], 148, [&](int ctas) { return ctas <= limit; });
       if (got != (want[i] < limit ? want[i] : limit)) return printf("%d %d: %d\n", i, limit, got), 1;
