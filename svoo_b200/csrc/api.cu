@@ -313,7 +313,8 @@ static int sparse_attn_impl(bool tensor_core, const void* q, const void* k, cons
   int32_t* head_order = ws_at<int32_t>(workspace, w.head_order);
   int32_t* sched = ws_at<int32_t>(workspace, w.sched);
   int32_t* status = ws_at<int32_t>(workspace, w.status);            // word 0: attention kernel
-  SVOO_CUDA(cudaMemsetAsync(sched, 0, (size_t)(w.status - w.sched) + 4, st));
+  // the status word behind `sched` belongs to the tcgen05 kernels
+  SVOO_CUDA(cudaMemsetAsync(sched, 0, (size_t)(w.status - w.sched) + (tensor_core ? 4 : 0), st));
   SVOO_CUDA(launch_attn_lists(q_offsets, qtiles, nqtiles, map, k_offsets, runs, nruns, sched, head_order, BH, S, QC, KC, max_runs(KC),
                               tensor_core ? 256 : 128, tensor_core && single_tile_kernel_wins(S, QC, false), false, st));
   if (tensor_core) {

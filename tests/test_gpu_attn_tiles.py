@@ -173,3 +173,23 @@ def test_single_tiles_are_the_same_in_either_kernel(name, ear):
         else:
             got.append(ops.sparse_attn(q, k, v, m, q_off, k_off, return_lse=True))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+def test_status_word_is_the_tensor_core_kernels_own():
+    """The status word tells of the last tcgen05 call that used the workspace: that call clears it, the mma.sync
+    cross-check leaves it alone."""
+    import ctypes
+    from svoo_b200 import ops
+    from svoo_b200._lib import LIB
+    dev = torch.device("cuda")
+    H, S, QC, KC = 2, 300, 3, 4
+    q, k, v = (torch.randn(H, S, 128, device=dev).to(torch.bfloat16) for _ in range(3))
+    args = (torch.ones(H, QC, KC, dtype=torch.uint8, device=dev), _offsets(torch.tensor([[100] * QC] * H), dev),
+            _offsets(torch.tensor([[75] * KC] * H), dev))
+    off = ctypes.c_int64(0)
+    assert LIB.svoo_b200_status_offset(H, S, QC, KC, ctypes.byref(off)) == 0
+    ops.workspace(dev, H, S, QC, KC)[off.value] = 1               # as a kernel that gave up would leave it
+    ops.sparse_attn(q, k, v, *args, kernel="simt")
+    assert ops.attention_status(dev, H, S, QC, KC) == 1
+    ops.sparse_attn(q, k, v, *args)
+    assert ops.attention_status(dev, H, S, QC, KC) == 0
