@@ -28,7 +28,7 @@
 extern "C" {
 #endif
 
-#define SVOO_B200_VERSION 104
+#define SVOO_B200_VERSION 105
 
 enum {
   SVOO_OK = 0,

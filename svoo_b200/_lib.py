@@ -84,7 +84,7 @@ SIGNATURES = {
 }
 
 
-VERSION = 104          # SVOO_B200_VERSION of include/svoo_b200.h this binding was written for
+VERSION = 105          # SVOO_B200_VERSION of include/svoo_b200.h this binding was written for
 
 
 class SvooB200Error(RuntimeError):
