@@ -8,7 +8,7 @@ cudaError_t launch_prologue(const void*, const void*, void*, void*, int64_t, int
 cudaError_t launch_assign_tc(const void*, int64_t, const void*, const void*, int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
 int assign_groups(int64_t J);
 cudaError_t launch_assign_reduce(const int2*, int32_t*, int64_t, int64_t, int64_t, cudaStream_t);
-cudaError_t launch_sort_labels(const int2*, int, int32_t*, int64_t, int64_t, int64_t, int32_t*, int32_t*, int32_t*, cudaStream_t);
+cudaError_t launch_sort_labels(const int2*, int, int32_t*, int64_t, int64_t, int64_t, int32_t*, int32_t*, cudaStream_t);
 cudaError_t launch_centroid_update(const void*, int64_t, const int32_t*, const int32_t*, const void*, void*, int32_t*, float*,
                                    int64_t, int64_t, int64_t, cudaStream_t);
 cudaError_t launch_offsets_from_sizes(const int32_t*, int32_t*, int64_t, int64_t, cudaStream_t);
@@ -157,8 +157,7 @@ int svoo_b200_sort_labels(const int32_t* labels, int64_t BH, int64_t N, int64_t 
   SVOO_TRY(check_clusters(K));
   const Workspace w = workspace_layout(BH, N, K, K);
   if (workspace_bytes < w.total) return SVOO_ERR_WORKSPACE;
-  SVOO_CUDA(launch_sort_labels(nullptr, 0, const_cast<int32_t*>(labels), BH, N, K, sorted_idx, offsets, nullptr,
-                               (cudaStream_t)stream));
+  SVOO_CUDA(launch_sort_labels(nullptr, 0, const_cast<int32_t*>(labels), BH, N, K, sorted_idx, offsets, (cudaStream_t)stream));
   return SVOO_OK;
 }
 
@@ -212,12 +211,12 @@ int svoo_b200_cocluster_rows(const void* q, const void* k, const int32_t* q_init
     // keys: profile over the query centroids
     SVOO_CUDA(launch_prologue(kcentroids, qcentroids, w_hi, w_lo, BH, KC, QC, st));
     SVOO_CUDA(launch_assign_tc(k, head_rows, w_hi, w_lo, apart, status, BH, N, KC, st));
-    SVOO_CUDA(launch_sort_labels(apart, assign_groups(KC), klabels, BH, N, KC, k_sorted_idx, k_offsets, nullptr, st));
+    SVOO_CUDA(launch_sort_labels(apart, assign_groups(KC), klabels, BH, N, KC, k_sorted_idx, k_offsets, st));
     SVOO_CUDA(launch_centroid_update(k, head_rows, k_sorted_idx, k_offsets, kcentroids, kcentroids, ksizes, partial, BH, N, KC, st));
     // queries: profile over the just-updated key centroids
     SVOO_CUDA(launch_prologue(qcentroids, kcentroids, w_hi, w_lo, BH, QC, KC, st));
     SVOO_CUDA(launch_assign_tc(q, head_rows, w_hi, w_lo, apart, status, BH, N, QC, st));
-    SVOO_CUDA(launch_sort_labels(apart, assign_groups(QC), qlabels, BH, N, QC, q_sorted_idx, q_offsets, nullptr, st));
+    SVOO_CUDA(launch_sort_labels(apart, assign_groups(QC), qlabels, BH, N, QC, q_sorted_idx, q_offsets, st));
     SVOO_CUDA(launch_centroid_update(q, head_rows, q_sorted_idx, q_offsets, qcentroids, qcentroids, qsizes, partial, BH, N, QC, st));
   }
   return SVOO_OK;

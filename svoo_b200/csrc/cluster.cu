@@ -266,8 +266,8 @@ __device__ __forceinline__ unsigned same_label(int label, bool ok, int bits) {
 
 template <int kGroups>
 __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kernel(
-    const int2* __restrict__ partial, int32_t* labels, int32_t* __restrict__ sorted_idx, int32_t* __restrict__ offsets,
-    int32_t* __restrict__ sizes, int BH, int N, int K) {
+    const int2* __restrict__ partial, int32_t* labels, int32_t* __restrict__ sorted_idx, int32_t* __restrict__ offsets, int BH,
+    int N, int K) {
   extern __shared__ int sort_sm[];
   int* wh = sort_sm;                                     // [16][K] counts, then positions, per warp
   int* tot = wh + kSortWarps * K;                        // [K] this CTA's totals, then the head's
@@ -406,10 +406,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_labels_kern
     const int k = tid * per + u;
     if (u < per && k < K) {
       add[k] = excl + before[u];
-      if (rank == 0) {
-        offsets[(int64_t)bh * (K + 1) + k] = excl;
-        if (sizes) sizes[(int64_t)bh * K + k] = all[u];
-      }
+      if (rank == 0) offsets[(int64_t)bh * (K + 1) + k] = excl;
     }
     excl += all[u];
   }
@@ -603,7 +600,7 @@ cudaError_t launch_prologue(const void* own, const void* form, void* w_hi, void*
 // Whether the device can place a cluster of `ctas` CTAs of the sort with the shared memory of the most clusters: sizes
 // above 8 are not portable, and a partition of a GPU has fewer SMs to a GPC.  Asked once per device, kernel form
 // and size; the answer is the device's.
-using SortKernel = void (*)(const int2*, int32_t*, int32_t*, int32_t*, int32_t*, int, int, int);
+using SortKernel = void (*)(const int2*, int32_t*, int32_t*, int32_t*, int, int, int);
 static bool sort_cluster_fits(SortKernel kernel, int form, int dev, int ctas) {
   constexpr int kDevices = 64;
   static std::atomic<signed char> known[kDevices][5][5];                     // [log2 ctas]: 0 not asked, 1 yes, -1 no
@@ -631,7 +628,7 @@ static bool sort_cluster_fits(SortKernel kernel, int form, int dev, int ctas) {
 
 // groups > 0: `labels` are first reduced from that many column groups of `partial` (see assign_tc.cu).
 cudaError_t launch_sort_labels(const int2* partial, int groups, int32_t* labels, int64_t BH, int64_t N, int64_t K,
-                               int32_t* sorted_idx, int32_t* offsets, int32_t* sizes, cudaStream_t st) {
+                               int32_t* sorted_idx, int32_t* offsets, cudaStream_t st) {
   SortKernel kernel = nullptr;
   switch (groups) {                                      // two per 256 (at most 128 clusters: 128) W rows
     case 0: kernel = sort_labels_kernel<0>; break;
@@ -663,7 +660,7 @@ cudaError_t launch_sort_labels(const int2* partial, int groups, int32_t* labels,
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   count_launches(1);
-  return cudaLaunchKernelEx(&cfg, kernel, partial, labels, sorted_idx, offsets, sizes, (int)BH, (int)N, (int)K);
+  return cudaLaunchKernelEx(&cfg, kernel, partial, labels, sorted_idx, offsets, (int)BH, (int)N, (int)K);
 }
 
 cudaError_t launch_centroid_update(const void* x, int64_t x_head_rows, const int32_t* sorted_idx, const int32_t* offsets,
@@ -706,7 +703,6 @@ extern "C" int svoo_b200_sort_labels_static(const int32_t* labels, int64_t BH, i
   if (BH < 1 || BH > 65535 || N < 1 || N > (1 << 24) || K < 1 || BH * N > (int64_t)INT32_MAX) return SVOO_ERR_SHAPE;
   if (K > SVOO_MAX_CLUSTERS) return SVOO_ERR_CLUSTERS;
   if (BH * ceil_div64(N, kCountChunk) * K > kMaxCounts) return SVOO_ERR_STATIC_SCRATCH;
-  cudaError_t e = launch_sort_labels(nullptr, 0, const_cast<int32_t*>(labels), BH, N, K, sorted_idx, offsets, nullptr,
-                                     (cudaStream_t)stream);
+  cudaError_t e = launch_sort_labels(nullptr, 0, const_cast<int32_t*>(labels), BH, N, K, sorted_idx, offsets, (cudaStream_t)stream);
   return e == cudaSuccess ? SVOO_OK : (int)e;
 }
