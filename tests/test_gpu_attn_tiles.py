@@ -188,7 +188,7 @@ def test_status_word_is_the_tensor_core_kernels_own():
             _offsets(torch.tensor([[75] * KC] * H), dev))
     off = ctypes.c_int64(0)
     assert LIB.svoo_b200_status_offset(H, S, QC, KC, ctypes.byref(off)) == 0
-    ops.workspace(dev, H, S, QC, KC)[off.value] = 1               # as a kernel that gave up would leave it
+    ops.workspace(dev, H, S, QC, KC)[off.value:off.value + 4].view(torch.int32).fill_(1)       # as a kernel that gave up
     ops.sparse_attn(q, k, v, *args, kernel="simt")
     assert ops.attention_status(dev, H, S, QC, KC) == 1
     ops.sparse_attn(q, k, v, *args)
