@@ -166,7 +166,10 @@ class _SAPBase:
     # the transpose behind it a view
     _token_major = False
 
-    def _sparse(self, query, key, value, prompt_length=None):
+    def _sparse(self, query, key, value, prompt_length=None, token_major=None):
+        """[1, H, S, 128], contiguous or (`token_major`) a view of contiguous [1, S, H, 128] rows."""
+        if token_major is None:
+            token_major = self._token_major
         cfg, H, S, D = query.shape
         n_video = self.num_frame * self.frame_size
         qv, kv = (query[:, :, :n_video], key[:, :, :n_video]) if self.context_length else (query, key)
@@ -175,7 +178,7 @@ class _SAPBase:
         self._last_shape = (query.device, cfg * H, S, n_video, self.num_q_centroids + extra, self.num_k_centroids + extra)
         ratio = self._get_min_kc_ratio_for_heads_from_step(self.current_inference_step, H)
         rows, peer_out = None, None
-        if self._token_major and cfg == 1 and H <= 128:
+        if token_major and cfg == 1 and H <= 128:
             rows = torch.empty(cfg, S, H, D, dtype=query.dtype, device=query.device)
             peer_out = ops.token_major(rows)
         out, state = sparse_attention_layer(query, key, value, num_q_centroids=self.num_q_centroids,
@@ -444,12 +447,22 @@ class Hunyuan_SAPAttn_Processor2_0(_SAPBase):
             query, key = self.get_rotary_emb(attn, query, key, image_rotary_emb, encoder_hidden_states)
             query, key, value = self.get_encoder_condition_and_concat(attn, query, key, value, encoder_hidden_states)
         cu_max_seqlens = None if attention_mask is None else self.get_cu_max_seqlen(attention_mask, query.device)
-        hidden_states = self.attention_core_logic(query, key, value, timestep, self.layer_idx, cu_max_seqlens)
+        # an own attention_core_logic (a subclass, a patched instance) is called; otherwise the rows may stay
+        # token-major, which makes the transpose a view
+        if getattr(self.attention_core_logic, "__func__", None) is Hunyuan_SAPAttn_Processor2_0._stock_core_logic:
+            hidden_states = self._core(query, key, value, timestep, cu_max_seqlens, token_major=True)
+        else:
+            hidden_states = self.attention_core_logic(query, key, value, timestep, self.layer_idx, cu_max_seqlens)
         hidden_states = hidden_states.transpose(1, 2).flatten(2, 3).to(query.dtype)
         return self.get_o(attn, hidden_states, encoder_hidden_states)
 
     def attention_core_logic(self, query, key, value, timestep, layer_idx=None, cu_max_seqlens=None):
-        """query/key/value [1, H, S, 128] -> [1, H, S, 128] (hunyuan10/attention.py:1031-1110)."""
+        """query/key/value [1, H, S, 128] -> contiguous [1, H, S, 128] (hunyuan10/attention.py:1031-1110)."""
+        return self._core(query, key, value, timestep, cu_max_seqlens, token_major=False)
+
+    _stock_core_logic = attention_core_logic
+
+    def _core(self, query, key, value, timestep, cu_max_seqlens, token_major):
         cfg, H, S, D = query.size()
         assert cfg == 1, "Batch size must be 1 for kmeans block sparse attention"
         assert 0 <= self.prompt_length <= self.context_length, "prompt_length must lie in [0, context_length]"
@@ -468,4 +481,4 @@ class Hunyuan_SAPAttn_Processor2_0(_SAPBase):
             if valid < S:
                 out[:, :, valid:] = self.flash_attention(query[:, :, valid:], key[:, :, valid:], value[:, :, valid:])
             return out
-        return self._sparse(query, key, value, prompt_length=self.prompt_length)
+        return self._sparse(query, key, value, prompt_length=self.prompt_length, token_major=token_major)

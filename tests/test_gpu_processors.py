@@ -441,3 +441,44 @@ def test_core_logic_results_are_contiguous(dev, name, timestep):
     assert out.shape == ((1, H, S, 128) if joint else (1, S, H * 128))
     assert out.is_contiguous() and out.dtype == q.dtype
     out.view(-1, 128)
+
+
+@pytest.mark.parametrize("how", ["subclass", "instance"])
+def test_hunyuan_call_uses_an_own_core_logic(dev, how):
+    """__call__ goes through attention_core_logic where that is replaced, with the result of the stock call, bit for bit."""
+    from svoo_b200 import processor
+    z = gu.load("processor_hunyuan")
+    P = gu.HUN_PROC
+    cls = _fresh(processor.Hunyuan_SAPAttn_Processor2_0)
+    gu.configure_hunyuan_processor(cls)
+    attn = gu.make_attn(41, P["heads"], joint=True).to(dev)
+    hidden, enc, mask = (t.to(dev) for t in gu.hunyuan_inputs())
+    step, tval = P["steps"][0]
+    qi, ki = torch.from_numpy(z["q_init"]).long().to(dev), torch.from_numpy(z["k_init"]).long().to(dev)
+    seen = []
+
+    class Own(cls):
+        def attention_core_logic(self, *a, **kw):
+            out = super().attention_core_logic(*a, **kw)
+            seen.append(out.view(-1, 128).shape)                  # contiguous
+            return out
+
+    def run(proc):
+        proc._step_from_callback = step
+        proc.draw_init_indices = lambda BH, n, d: (qi, ki)
+        with torch.no_grad():
+            return proc(attn, hidden, encoder_hidden_states=enc, attention_mask=mask, image_rotary_emb=None,
+                        timestep=torch.tensor([tval], device=dev))
+
+    want = run(cls(0))
+    assert not seen
+    if how == "subclass":
+        proc = Own(0)
+    else:
+        proc = cls(0)
+        inner = proc.attention_core_logic
+        proc.attention_core_logic = lambda *a, **kw: seen.append(None) or inner(*a, **kw)
+    got = run(proc)
+    assert len(seen) == 1
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
