@@ -258,9 +258,11 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
     };
     // 128 keys: both steps' maxima decide on the maximum before any of their P goes to the tensor core.  It rarely
     // changes after the first 128 keys, so the first step's P is computed on the old one while the second step's S is
-    // still being formed, kept in registers, and computed again if the maximum did change.
+    // still being formed, kept in registers, and computed again if the maximum did change.  Whether the first step changes
+    // it is looked at only where its P add up to more than 250: one above 2^8 would.
     for (int j0 = 0; j0 < T; j0 += 2) {
       const uint32_t par = (j0 >> 1) & 1;
+      const int n = min(T - j0, 2);
       uint32_t pk[32];
       uint64_t acc = 0;                                           // two fp32 zeros
       float m0 = -INFINITY, m1 = -INFINITY;
@@ -268,17 +270,21 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
       if (!ok) break;
       tc_fence_after();
       bool have_p = j0 > 0;
-      quarters(j0, [&](int c, const uint32_t (&x)[16]) {
-        max16(x, m0, m1);
-        if (have_p) have_p = !__any_sync(0xffffffffu, lane_has_row && fmaxf(m0, m1) * scale_log2 > m_used + kRescaleThreshold);
-        if (have_p) exp_pack16(x, &pk[c * 8], scale2, pair2(-m_used), acc);
-      });
-      if (j0 + 1 < T) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(SM_S_FULL + 1), par, abort_flag));
-        if (!ok) break;
-        tc_fence_after();
-        quarters(j0 + 1, [&](int, const uint32_t (&x)[16]) { max16(x, m0, m1); });
+      int u0 = 0;                                                 // steps [u0, n) are searched for their maximum
+      if (have_p) {
+        quarters(j0, [&](int c, const uint32_t (&x)[16]) { exp_pack16(x, &pk[c * 8], scale2, pair2(-m_used), acc); });
+        u0 = __any_sync(0xffffffffu, lane_has_row && !(pair_sum(acc) <= 250.f)) ? 0 : 1;
       }
+#pragma unroll 1
+      for (int u = u0; u < n; ++u) {
+        if (u == 1) {
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(SM_S_FULL + 1), par, abort_flag));
+          if (!ok) break;
+          tc_fence_after();
+        }
+        quarters(j0 + u, [&](int, const uint32_t (&x)[16]) { max16(x, m0, m1); });
+      }
+      if (!ok) break;
       const float m_tile = fmaxf(m0, m1) * scale_log2;            // the scale is positive
       if (j0 == 0) {
         m_used = kEar ? fmaxf(m_tile, -1e30f) : m_tile;           // EAR: first steps of masked centroids only
@@ -316,15 +322,16 @@ __global__ void __launch_bounds__(kSmThreads, 2) sparse_attn_small_kernel(
       else
         acc = 0;
 #pragma unroll 1
-      for (int u = have_p ? 1 : 0; u < min(T - j0, 2); ++u) {
+      for (int u = have_p ? 1 : 0; u < n; ++u) {
         quarters(j0 + u, [&](int c, const uint32_t (&x)[16]) { exp_pack16(x, &pk[c * 8], scale2, negm2, acc); });
         hand_over(u);
       }
       l_sum += pair_sum(acc);
     }
     // epilogue: O / l -> bf16 rows
-    const int row = row0 + r_local;
-    const bool store = lane_has_row && row < row1;
+    const int4 mine = __ldg(qtiles + (int64_t)bh * max_tiles + (max_tiles - QC) + t);     // again: registers are short above
+    const int row = mine.y + r_local;
+    const bool store = lane_has_row && row < mine.z;
     int dst = row;
     if (store && out_row_idx) dst = out_row_idx[(int64_t)bh * S + row];
     dst = store ? min(max(dst, 0), S - 1) : 0;
