@@ -315,7 +315,7 @@ static int sparse_attn_impl(bool tensor_core, const void* q, const void* k, cons
   // the status word behind `sched` belongs to the tcgen05 kernels
   SVOO_CUDA(cudaMemsetAsync(sched, 0, (size_t)(w.status - w.sched) + (tensor_core ? 4 : 0), st));
   SVOO_CUDA(launch_attn_lists(q_offsets, qtiles, nqtiles, map, k_offsets, runs, nruns, sched, head_order, BH, S, QC, KC, max_runs(KC),
-                              tensor_core ? 256 : 128, tensor_core && single_tile_kernel_wins(S, QC, false), false, st));
+                              tensor_core ? 256 : 128, tensor_core && single_tile_kernel_wins(S, QC, KC, false), false, st));
   if (tensor_core) {
     SVOO_CUDA(launch_sparse_attn_tc(q, k, v, out, out_row_idx, qtiles, nqtiles, head_order, runs, nruns, status, BH, S, QC,
                                     KC, sm_scale, peer_dst, my_heads, world, n_loc, H, lse, st));
@@ -467,7 +467,7 @@ static int sparse_attn_ear_impl(const void* q, const void* k_ext, const void* v_
   int32_t* status = ws_at<int32_t>(ear_workspace, w.status);
   SVOO_CUDA(cudaMemsetAsync(sched, 0, (size_t)(w.status - w.sched) + 4, st));
   SVOO_CUDA(launch_attn_lists(q_offsets, qtiles, nqtiles, map, k_offsets, runs, nruns, sched, head_order, BH, S, QC, KC, ear_max_runs(KC), 256,
-                              single_tile_kernel_wins(S, QC, true), true, st));
+                              single_tile_kernel_wins(S, QC, KC, true), true, st));
   SVOO_CUDA(launch_sparse_attn_tc(q, k_ext, v_ext, out, out_row_idx, qtiles, nqtiles, head_order, runs, nruns, status, BH, S, QC,
                                   KC, sm_scale, peer_dst, my_heads, world, n_loc, H, lse, st, map, k_offsets, ear_max_runs(KC)));
   return SVOO_OK;

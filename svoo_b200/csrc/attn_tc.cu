@@ -555,7 +555,7 @@ cudaError_t launch_sparse_attn_tc(const void* q, const void* k, const void* v, v
   const float scale_log2 = sm_scale * 1.4426950408889634f;
   const int runs_per_row = ear ? ear_max_runs : max_runs(KC);
   if (peer_dst) lse = nullptr;
-  const bool split = single_tile_kernel_wins(S, QC, ear);
+  const bool split = single_tile_kernel_wins(S, QC, KC, ear);
   // tiles per head: of at least 129 rows each, or a cluster's whole 256-row tiles and its remainder
   const int per_head = (int)(split ? S / (tc::kBM + 1) : S / (2 * tc::kBM) + QC);
   if (per_head > 0) {

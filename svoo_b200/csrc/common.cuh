@@ -48,13 +48,15 @@ __host__ inline int max_qtiles(int64_t N, int64_t QC) { return (int)(ceil_div64(
 //   60 rows per query cluster   12 x 32,760 tokens 0.64 / 0.86 / 0.90   12 x 12,150 0.53 / 0.78 / 0.83   2 x 32,760 0.64 / 0.83 / 0.87
 //   130                                     0.85 / 1.01 / 1.06                      0.83 / 0.94 / 1.00              0.84 / 0.98 / 0.99
 //   200                                     0.94 / 1.02 / 1.01                      0.99 / 1.03 / 1.04              1.10 / 1.20 / 1.23
-// With error-aware routing (every list ends with one long run of centroid keys) the two meet earlier: at 130 rows 0.96 / 1.02 / 1.04,
-// 0.90 / 1.00 / 1.04, 0.89 / 1.03 / 1.02.
-__host__ inline bool single_tile_kernel_wins(int64_t S, int64_t QC, bool ear) { return S < (ear ? 100 : 150) * QC; }
+// With error-aware routing (every list ends with one long run of centroid keys) the two meet earlier, except where the token
+// runs are short: at 130 rows 0.96 / 1.02 / 1.04, 0.90 / 1.00 / 1.04, 0.89 / 1.03 / 1.02.
 // The pair kernel gathers key tiles of many short runs with cp.async below 42 rows per key cluster.  With over without,
 // same tokens: 0.85 to 0.97 at 32 rows, 1.01 to 1.06 at 45 (finding out costs more than the boxes that are saved); a whole
 // Wan block of 12 x 20,280 tokens at 41 rows 2010 -> 1993 us.
 __host__ inline bool short_key_runs(int64_t S, int64_t KC) { return S < 42 * KC; }
+__host__ inline bool single_tile_kernel_wins(int64_t S, int64_t QC, int64_t KC, bool ear) {
+  return S < (ear && !short_key_runs(S, KC) ? 100 : 150) * QC;
+}
 
 // CTAs per head (one cluster) of the label sort: as many as surely fit the chip at once (a cluster stays inside one
 // GPC, so the last quarter of the slots is not counted on), of at least 512 tokens and K (a CTA clears and scans 16 K
