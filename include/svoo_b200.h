@@ -111,7 +111,8 @@ int svoo_b200_euclid_assign(const void* x, const void* centroids, int64_t BH, in
 
 /* Stable counting sort of labels in [0,K): sorted_idx[BH,N] and offsets[BH,K+1]
  * (replaces torch.argsort in svoo/kernels/triton/permute.py:90 and torch.sort in
- * svoo/co_clustering.py:274). */
+ * svoo/co_clustering.py:274).  The workspace is checked as for the other entry points; the sort itself
+ * keeps its counts in shared memory. */
 int svoo_b200_sort_labels(const int32_t* labels, int64_t BH, int64_t N, int64_t K,
                           int32_t* sorted_idx, int32_t* offsets,
                           void* workspace, int64_t workspace_bytes, void* stream);

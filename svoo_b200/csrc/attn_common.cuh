@@ -58,11 +58,12 @@ __device__ __forceinline__ void exp_pack16(const uint32_t (&r)[16], uint32_t* pk
   }
 }
 
-// CTA index -> (head, tile of the head's list).  The last kHoist tiles of every head go first: with text
-// tokens these are the prompt's query tiles, which attend to every key (720p HunyuanVideo: 930 key tiles
-// against 160 on average) and would otherwise be started last.  After them the heads follow one another,
-// so that the CTAs in flight share a head's K and V in L2, by decreasing work, so that the last CTAs are
-// short ones.  counts: (pairs, singles) of every head.
+// CTA index -> (head, tile of the head's list).  The last kHoist tiles of every head's list go first.  Tiles are in
+// cluster order and the text blocks come last, so where the whole text is prompt these are the prompt's query tiles,
+// which attend to every key (720p HunyuanVideo: 930 key tiles against 160 on average) and would otherwise be started
+// last.  A partly used prompt whose unused rows have a tile in the same list keeps its place at the end of the
+// head.  After them the heads follow one another, so that the CTAs in flight share a head's K and V in L2, by
+// decreasing work, so that the last CTAs are short ones.  counts: (pairs, singles) of every head.
 template <int kHoist>
 __device__ __forceinline__ bool pick_tile(int id, int BH, int per_head, const int32_t* counts, const int32_t* order, int which,
                                           int& bh, int& t) {

@@ -546,7 +546,8 @@ cudaError_t launch_append_text_blocks(const uint8_t* map, const int32_t* q_off, 
   return cudaGetLastError();
 }
 
-// A grid of up to 256 query clusters starts in one wave, whatever the order of the heads.
+// The heads are ordered by work above 256 query clusters in all: below that the call is small, or has a few heads of
+// many tokens, whose tiles then run in the order of the heads.
 // tile_rows: 128 (mma.sync kernel) or 256; split: single tiles in their own list.  ear: with the head's
 // centroid run (256-row tiles only).
 cudaError_t launch_attn_lists(const int32_t* q_offsets, int4* qtiles, int32_t* nqtiles, const uint8_t* map,
